@@ -131,6 +131,7 @@ void PWGrid::build(const PWBasisK& b) {
             km.h_precond[g] = 1.0 + g2 + std::sqrt(1.0 + (g2 - 1.0) * (g2 - 1.0));
         }
     }
+    build_line_plan(*this);
 }
 
 void PWGrid::ensure_device() {
@@ -143,6 +144,7 @@ void PWGrid::ensure_device() {
     st_ixy.upload(h_sixy.data(), nst);
     xpos.upload(h_xpos.data(), nxc);
     smap.upload(h_smap.data(), h_smap.size());
+    if (lines.ok) cdesc.upload(h_cdesc.data(), h_cdesc.size());
     const size_t L = size_t(basis.npwk_max);
     for (int ik = 0; ik < basis.nks; ++ik) {
         KMap& km = kmaps[ik];
@@ -150,6 +152,7 @@ void PWGrid::ensure_device() {
         km.gofs.upload(km.h_gofs.data(), nst + 1);
         km.gpk.upload(km.h_gpk.data(), npw);
         km.glist.upload(km.h_glist.data(), npw);
+        if (lines.ok) km.sd.upload(km.h_sd.data(), km.h_sd.size());
         km.ig2ixyz.upload(&basis.ig2ixyz_k[ik * L], npw);
         km.gk2.upload(&basis.gk2[ik * L], npw);
         std::vector<float> gf(npw);
@@ -529,9 +532,10 @@ void launch_hpsi_local(const PWGrid& g, int ik, const R* veff_zyx, const R* veff
                        T* hpsi, T* stickbuf, double tpiba2, int accumulate, cudaStream_t s) {
     if (nb <= 0) return;
     B200_CHECK(nb <= 65535, kInvalidArgument, "too many bands in one launch");
-    // compile-time warp transforms for the standard grid sizes; generic Stockham kernels otherwise
-    if (launch_hpsi_local_fast<T, R>(g, ik, veff_zyx, veff_perm, nb, ld, psi, hpsi, stickbuf, tpiba2, accumulate, s))
-        return;
+    // register transforms of the 64-, 96- and 128-point grids, line transforms of the others; the Stockham kernels
+    // below take what neither covers (an edge without two factors of the line transforms, a plane too large)
+    if (launch_hpsi_local_fast<T, R>(g, ik, veff_perm, nb, ld, psi, hpsi, stickbuf, tpiba2, accumulate, s)) return;
+    if (launch_hpsi_local_lines<T, R>(g, ik, veff_zyx, nb, ld, psi, hpsi, stickbuf, tpiba2, accumulate, s)) return;
     const size_t zs = zpass_smem(g, sizeof(T));
     const size_t ps = plane_smem(g, sizeof(T));
     B200_CHECK(ps <= 227 * 1024, kCapacityError, "plane pass does not fit in shared memory for this grid");
@@ -560,6 +564,7 @@ void launch_hpsi_local_nc(const PWGrid& g, int ik, const R* veff4_zyx, int ncols
                           T* stickbuf, T* rbuf, double tpiba2, cudaStream_t s) {
     if (ncols <= 0) return;
     B200_CHECK(ncols <= 65535 && ncols % 2 == 0, kInvalidArgument, "npol = 2: an even number of spinor columns, at most 65535");
+    if (launch_hpsi_local_nc_lines<T, R>(g, ik, veff4_zyx, ncols, ld, psi, hpsi, stickbuf, tpiba2, s)) return;
     const size_t zs = zpass_smem(g, sizeof(T));
     const size_t ps = plane_smem(g, sizeof(T));
     B200_CHECK(ps <= 227 * 1024, kCapacityError, "plane pass does not fit in shared memory for this grid");

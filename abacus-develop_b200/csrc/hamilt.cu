@@ -438,16 +438,18 @@ void Hamilt::hpsi_nc(int ik, int nb, int ld, const T* psi, T* hpsi, cudaStream_t
     B200_CHECK(nb >= 0 && ld >= npw, kInvalidArgument, "ld smaller than npwk or negative band count");
     B200_CHECK(has_veff_nc, kInvalidArgument, "npol = 2: V_eff's four components not set");
     if (nb == 0) return;
-    // local part, in chunks of bands whose real-space planes (two boxes per band) stay within 512 MB
+    // local part, in chunks of bands whose scratch stays within 512 MB: the stick buffer where both components' planes
+    // fit in shared memory, else two real-space boxes per band as well
     const size_t N = size_t(grid->nxyz());
-    const size_t per_col = N * sizeof(T);
+    const bool fused = lines_supported(*grid, sizeof(T), 2);
+    const size_t per_col = (fused ? size_t(grid->nst) * grid->nz : N) * sizeof(T);
     int cb = int((size_t(512) << 20) / (2 * per_col));
     if (cb < 1) cb = 1;
     if (cb > nb) cb = nb;
     if (cb > 32767) cb = 32767;
     const R* v4 = f64 ? (const R*)veff_nc_zyx.ptr : (const R*)veff_nc_zyxf.ptr;
     T *sb, *rb;
-    const size_t sbn = size_t(2) * cb * grid->nst * grid->nz, rbn = size_t(2) * cb * N;
+    const size_t sbn = size_t(2) * cb * grid->nst * grid->nz, rbn = fused ? 0 : size_t(2) * cb * N;
     if constexpr (f64) {
         W.sb64.resize(sbn);
         W.rb64.resize(rbn);

@@ -1,0 +1,107 @@
+// Launch of the plane pass on line transforms (plane_g.cuh): run-time geometry, or the x line (and on square planes
+// the y line) compiled in.  Compiled lines take about half the instructions of run-time ones (no index arithmetic, no
+// dispatch), and their code stays in the instruction cache.
+#pragma once
+#include "plane_g.cuh"
+
+namespace b200 {
+namespace line {
+
+// threads of a CTA, and resident threads of an SM, by the registers the transforms need: FP64 lines of 12 points and
+// more in pass A take 168 a thread (96^2: 12 warps of 168 run the local pass in 1.53 ms, 16 of 128 in 1.56)
+constexpr int plane_threads(size_t elem, int r1) { return elem == 8 || r1 <= 10 ? 512 : r1 <= 16 ? 384 : 256; }
+
+template <typename T> const T* roots_of(const FftAxis& a) {
+    if constexpr (sizeof(T) == 16) return a.rt64.ptr;
+    else return a.rt32.ptr;
+}
+template <typename K> void set_smem(K kernel, size_t bytes) {
+    if (bytes > 48 * 1024) B200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
+}
+
+template <typename T, typename R, int RMAX, int NPOL, typename GX, typename GY>
+void plane_launch(const PWGrid& g, const PlaneShape& sh, int nplanes, GX gx, GY gy, const R* v, T* sb, cudaStream_t s) {
+    auto kern = k_plane_g<T, R, RMAX, NPOL, plane_threads(sizeof(T), RMAX), GX, GY>;
+    set_smem(kern, sh.smem);
+    kern<<<dim3(nplanes, g.nz), sh.nw * 32, sh.smem, s>>>(g.plane_view(), gx, gy, sh.L, g.nz, roots_of<T>(g.ax),
+                                                          roots_of<T>(g.ay), v, size_t(g.nxyz()), sb);
+    note_launch();
+    B200_CUDA(cudaGetLastError());
+}
+
+// the plane pass with x lines of N compiled in; false for other grids
+template <typename T, typename R, int N>
+bool plane_fixed(const PWGrid& g, const PlaneShape& sh, int nplanes, const R* v, T* sb, cudaStream_t s) {
+    if (g.nx != N) return false;
+    constexpr int elem = sizeof(T);
+    constexpr LineGeom x = x_geom(N, elem), y = y_geom(N, elem, x.r2);
+    using GX = FixedGeom<N, x.r1, x.r2, x.rs, x.ld>;
+    using GY = FixedGeom<N, y.r1, y.r2, y.rs, y.ld>;
+    constexpr int rmax = x.r1;
+    if (g.ny == N) {
+        plane_launch<T, R, rmax, 1>(g, sh, nplanes, GX(), GY(), v, sb, s);
+        return true;
+    }
+    const LineGeom& yd = g.lines.y[elem == 8];
+    if (yd.r1 > 16) return false;
+    if (rmax <= 10 && yd.r1 <= 10) plane_launch<T, R, (rmax <= 10 ? 10 : 16), 1>(g, sh, nplanes, GX(), yd, v, sb, s);
+    else plane_launch<T, R, (rmax > 16 ? rmax : 16), 1>(g, sh, nplanes, GX(), yd, v, sb, s);
+    return true;
+}
+
+// the z passes take one k-point (OneK) or a batch indexed by blockIdx.z (ManyK)
+struct OneK {
+    KBatchEntry e;
+    __device__ __forceinline__ const KBatchEntry& get(int) const { return e; }
+};
+struct ManyK {
+    KBatchArgs a;
+    __device__ __forceinline__ const KBatchEntry& get(int q) const { return a.e[q]; }
+};
+template <typename T, typename Src> struct ZArgs {
+    bool inv;
+    const Src& src;
+    int nk, b0, nbc;
+    T* sb;
+    double tpiba2;
+    int accumulate;
+    cudaStream_t s;
+};
+template <typename T> constexpr int z_tile() { return sizeof(T) == 16 ? 16 : 32; }  // 256 bytes of a plane row
+
+template <typename T, typename R, int RMAX, typename Src, typename GZ>
+void z_launch(const PWGrid& g, GZ gz, const ZArgs<T, Src>& a) {
+    constexpr int TS = z_tile<T>();
+    const size_t smem = size_t(TS) * gz.ld * sizeof(T);
+    const dim3 grid(ceil_div(g.nst, TS), a.nbc, a.nk);
+    if (a.inv) {
+        auto kern = k_zinv_g<T, RMAX, TS, Src, GZ>;
+        set_smem(kern, smem);
+        kern<<<grid, 128, smem, a.s>>>(a.src, gz, a.b0, a.nbc, roots_of<T>(g.az), a.sb);
+    } else {
+        auto kern = k_zfwd_g<T, R, RMAX, TS, Src, GZ>;
+        set_smem(kern, smem);
+        kern<<<grid, 128, smem, a.s>>>(a.src, gz, a.b0, a.nbc, roots_of<T>(g.az), a.sb, R(a.tpiba2),
+                                       R(1.0 / double(g.nxyz())), a.accumulate);
+    }
+    note_launch();
+    B200_CUDA(cudaGetLastError());
+}
+template <typename T, typename R, int N, typename Src> bool z_fixed_n(const PWGrid& g, const ZArgs<T, Src>& a) {
+    constexpr LineGeom z = z_geom(N, sizeof(T));
+    z_launch<T, R, z.r1>(g, FixedGeom<N, z.r1, z.r2, z.rs, z.ld>(), a);
+    return true;
+}
+// the z passes with lines of nz compiled in; false for other grids (zpass_f64.cu, zpass_f32.cu, and *_many)
+template <typename T, typename R, typename Src> bool z_fixed(const PWGrid& g, const ZArgs<T, Src>& a);
+
+// the compiled edges (2-, 3-, 5-smooth, 16 to 160), split over translation units
+template <typename T, typename R>
+bool plane_fixed_a(const PWGrid& g, const PlaneShape& sh, int nplanes, const R* v, T* sb, cudaStream_t s);
+template <typename T, typename R>
+bool plane_fixed_b(const PWGrid& g, const PlaneShape& sh, int nplanes, const R* v, T* sb, cudaStream_t s);
+template <typename T, typename R>
+bool plane_fixed_c(const PWGrid& g, const PlaneShape& sh, int nplanes, const R* v, T* sb, cudaStream_t s);
+
+}  // namespace line
+}  // namespace b200

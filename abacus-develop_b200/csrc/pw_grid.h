@@ -17,6 +17,7 @@
 
 #include "common.h"
 #include "fft_core.cuh"
+#include "line_plan.h"
 #include "pw_basis.h"
 
 namespace b200 {
@@ -46,6 +47,8 @@ struct KMap {
     DeviceArray<float> gk2f;
     DeviceArray<double> precond;  // Davidson preconditioner 1 + g2 + sqrt(1 + (g2-1)^2)
     DeviceArray<double> gkcar;    // k+G cartesian (npw x 3, units of tpiba): PW_Basis_K::getgpluskcar
+    std::vector<int2> h_sd;       // stick descriptors of the line transforms (StickMapView::sd)
+    DeviceArray<int2> sd;
 };
 
 // Index maps handed to kernels by value.
@@ -54,6 +57,7 @@ struct StickMapView {
     const int* gofs;
     const int* gpk;
     const int* glist;
+    const int2* sd;  // per stick (line transforms): first position in psi, first z | count << 16
 };
 struct PlaneMapView {
     int nst, nxc;
@@ -61,6 +65,27 @@ struct PlaneMapView {
     const int* sy;    // per stick: y
     const int* xpos;  // per compact column: x
     const int* smap;  // per compact column c and y < ny: the stick at (xpos[c], y), or -1 (nxc x ny)
+    // line transforms: the sticks of column c are those of y in [0, cd.y) and [cd.z, cd.w), from stick cd.x on;
+    // the occupied x are [0, xm) and [xh, nx), x >= xh in column x - xoff
+    const int4* cd;
+    int xm, xh, xoff;
+};
+
+// A launch shape of the plane pass on the line transforms: nw warps a CTA, L rows a warp at a time, `ctas` CTAs
+// resident on an SM, `work` the instructions of the busiest warp (estimate).
+struct PlaneShape {
+    int nw = 0, L = 0, ctas = 0;
+    double work = 0;
+    size_t smem = 0;
+};
+// The line transforms of a grid; [0]: FP64, [1]: FP32.  ok: every edge factors, and the occupied x, the y of each
+// column and the z of each stick are runs (a sphere's always are).  shapes[precision][npol - 1]: candidates, empty
+// where a plane does not fit in shared memory.
+struct LinePlan {
+    bool ok = false;
+    LineGeom x[2], y[2], z[2];
+    int xm = 0, xh = 0, xoff = 0;
+    std::vector<PlaneShape> shapes[2][2];
 };
 
 struct PWGrid {
@@ -70,6 +95,9 @@ struct PWGrid {
     DeviceArray<int> st_xc, st_y, xpos, st_ixy, smap;
     std::vector<int> h_xpos, h_xc, h_sy, h_sixy, h_smap;
     std::vector<KMap> kmaps;
+    LinePlan lines;
+    std::vector<int4> h_cdesc;
+    DeviceArray<int4> cdesc;
     bool on_device = false;
     // plane pass of the register transforms, per precision (0: default shape; see plane_launch_var)
     int plane_variant64 = 0, plane_variant32 = 0;
@@ -78,9 +106,12 @@ struct PWGrid {
     void ensure_device();           // uploads plans and maps on first device use
     StickMapView stick_view(int ik) const {
         const KMap& k = kmaps[ik];
-        return StickMapView{nst, nz, k.gofs.ptr, k.gpk.ptr, k.glist.ptr};
+        return StickMapView{nst, nz, k.gofs.ptr, k.gpk.ptr, k.glist.ptr, k.sd.ptr};
     }
-    PlaneMapView plane_view() const { return PlaneMapView{nst, nxc, st_xc.ptr, st_y.ptr, xpos.ptr, smap.ptr}; }
+    PlaneMapView plane_view() const {
+        return PlaneMapView{nst,      nxc,        st_xc.ptr, st_y.ptr, xpos.ptr,
+                            smap.ptr, cdesc.ptr, lines.xm,  lines.xh, lines.xoff};
+    }
     long nxyz() const { return long(nx) * ny * nz; }
 };
 
@@ -98,11 +129,11 @@ size_t plane_smem(const PWGrid& g, size_t elem);
 template <typename T, typename R>
 void launch_hpsi_local(const PWGrid& g, int ik, const R* veff_zyx, const R* veff_perm, int nb, int ld, const T* psi,
                        T* hpsi, T* stickbuf, double tpiba2, int accumulate, cudaStream_t s);
-// Same, with warp-synchronous compile-time transforms; returns false (launching nothing) for
-// grid sizes it does not cover.
+// Same, on the register transforms of the 64-, 96- and 128-point grids; returns false (launching nothing) for
+// other grids.
 template <typename T, typename R>
-bool launch_hpsi_local_fast(const PWGrid& g, int ik, const R* veff_zyx, const R* veff_perm, int nb, int ld,
-                            const T* psi, T* hpsi, T* stickbuf, double tpiba2, int accumulate, cudaStream_t s);
+bool launch_hpsi_local_fast(const PWGrid& g, int ik, const R* veff_perm, int nb, int ld, const T* psi, T* hpsi,
+                            T* stickbuf, double tpiba2, int accumulate, cudaStream_t s);
 // k-point batch: one entry per k (its stick maps, psi / hpsi with leading dimension ld, npwk, gk2 in the
 // precision of the call); passed by value so a launch needs no device-side argument buffer.
 constexpr int kMaxKBatch = 128;
@@ -121,6 +152,20 @@ struct KBatchArgs {
 template <typename T, typename R>
 bool launch_hpsi_local_kbatch(const PWGrid& g, const KBatchArgs& args, int nk, int nb, const R* veff_zyx,
                               const R* veff_perm, T* stickbuf, int chunk, double tpiba2, cudaStream_t s);
+// The line transforms of grid g (host; fills g.lines and the run descriptors of columns and sticks).
+void build_line_plan(PWGrid& g);
+// The three passes on the line transforms (fft_lines.cu); false (nothing launched) where g.lines does not hold or a
+// plane does not fit in shared memory.
+bool lines_supported(const PWGrid& g, size_t elem, int npol);
+template <typename T, typename R>
+bool launch_hpsi_local_lines(const PWGrid& g, int ik, const R* veff_zyx, int nb, int ld, const T* psi, T* hpsi,
+                             T* stickbuf, double tpiba2, int accumulate, cudaStream_t s);
+template <typename T, typename R>
+bool launch_hpsi_local_kbatch_lines(const PWGrid& g, const KBatchArgs& args, int nk, int nb, const R* veff_zyx,
+                                    T* stickbuf, int chunk, double tpiba2, cudaStream_t s);
+template <typename T, typename R>
+bool launch_hpsi_local_nc_lines(const PWGrid& g, int ik, const R* veff4_zyx, int ncols, int ld, const T* psi, T* hpsi,
+                                T* stickbuf, double tpiba2, cudaStream_t s);
 // Drop-in transforms (PW_Basis_K::recip_to_real / real_to_recip on the GPU), one band.
 // the local part of H|psi> for npol = 2 (Veff::act's spinor branch, veff_pw.cpp:73-104, with Ekinetic::act on both
 // components): ncols spinor columns (band b's components at columns 2b, 2b+1, pitch ld), the four V_eff
