@@ -528,13 +528,12 @@ template <typename K> static void set_smem(K kernel, size_t bytes) {
 }
 
 template <typename T, typename R>
-void launch_hpsi_local(const PWGrid& g, int ik, const R* veff_zyx, const R* veff_perm, int nb, int ld, const T* psi,
-                       T* hpsi, T* stickbuf, double tpiba2, int accumulate, cudaStream_t s) {
+void launch_hpsi_local(const PWGrid& g, int ik, const R* veff_zyx, int nb, int ld, const T* psi, T* hpsi,
+                       T* stickbuf, double tpiba2, int accumulate, cudaStream_t s) {
     if (nb <= 0) return;
     B200_CHECK(nb <= 65535, kInvalidArgument, "too many bands in one launch");
-    // register transforms of the 64-, 96- and 128-point grids, line transforms of the others; the Stockham kernels
-    // below take what neither covers (an edge without two factors of the line transforms, a plane too large)
-    if (launch_hpsi_local_fast<T, R>(g, ik, veff_perm, nb, ld, psi, hpsi, stickbuf, tpiba2, accumulate, s)) return;
+    // line transforms; the Stockham kernels below take what they do not cover (an edge without two of their factors, a
+    // plane too large for shared memory)
     if (launch_hpsi_local_lines<T, R>(g, ik, veff_zyx, nb, ld, psi, hpsi, stickbuf, tpiba2, accumulate, s)) return;
     const size_t zs = zpass_smem(g, sizeof(T));
     const size_t ps = plane_smem(g, sizeof(T));
@@ -650,12 +649,10 @@ void launch_transpose_veff(const PWGrid& g, const double* veff, R* out, cudaStre
     B200_CUDA(cudaGetLastError());
 }
 
-template void launch_hpsi_local<double2, double>(const PWGrid&, int, const double*, const double*, int, int,
-                                                 const double2*, double2*,
+template void launch_hpsi_local<double2, double>(const PWGrid&, int, const double*, int, int, const double2*, double2*,
                                                  double2*, double, int, cudaStream_t);
-template void launch_hpsi_local<float2, float>(const PWGrid&, int, const float*, const float*, int, int, const float2*,
-                                               float2*, float2*,
-                                               double, int, cudaStream_t);
+template void launch_hpsi_local<float2, float>(const PWGrid&, int, const float*, int, int, const float2*, float2*,
+                                               float2*, double, int, cudaStream_t);
 template void launch_hpsi_local_nc<double2, double>(const PWGrid&, int, const double*, int, int, const double2*,
                                                     double2*, double2*, double2*, double, cudaStream_t);
 template void launch_hpsi_local_nc<float2, float>(const PWGrid&, int, const float*, int, int, const float2*, float2*,

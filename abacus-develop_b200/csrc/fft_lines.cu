@@ -11,29 +11,35 @@ constexpr size_t kSmemMax = 227 * 1024;
 
 constexpr int kSMs = 148;
 
-// the shapes of the plane pass worth choosing from: for every (nw, L) that fits, the work of the busiest warp
-// from the operation counts; a shape is dropped if another has no more work and no fewer resident CTAs
-std::vector<PlaneShape> plane_shapes(const PWGrid& g, int prec, int npol) {
+// instructions of the busiest of nw warps with L rows at a time, from the operation counts (x transforms one way
+// only and no V_eff for inverse_only)
+double warp_work(const LineGeom& x, const LineGeom& y, int ncols, int npol, int nw, int L, bool inverse_only) {
+    const int na = 32 / x.r2, nb = 32 / x.r1, nya = 32 / y.r2, nyb = 32 / y.r1, ways = inverse_only ? 1 : 2;
+    const double ca = ways * line::dft_ops(x.r1) + 5 * ways * x.r1 + 40;
+    const double cb = npol * (ways * line::dft_ops(x.r2) + 6 * ways * (x.r2 - 1) + 10 * ways * x.r2);
+    const double cya = ways * line::dft_ops(y.r1) + 15 * ways * y.r1 + 40;
+    const double cyb = ways * line::dft_ops(y.r2) + 6 * ways * y.r2 + 10 * ways * y.r2;
+    const int groups = ceil_div(ceil_div(y.n, L), nw), cper = ceil_div(ncols, nw);
+    return groups * (ceil_div(npol * L, na) * ca + ceil_div(L, nb) * cb) + ceil_div(cper, nya) * cya +
+           ceil_div(cper, nyb) * cyb;
+}
+
+// the shapes worth choosing from: for every (nw, L) that fits, the work of the busiest warp; a shape is dropped if
+// another has no more work and no fewer resident CTAs.  extra: further shared memory of a CTA
+std::vector<PlaneShape> plane_shapes(const PWGrid& g, int prec, int npol, bool inverse_only, size_t extra) {
     const LineGeom &x = g.lines.x[prec], &y = g.lines.y[prec];
     const size_t elem = prec ? 8 : 16;
     const int maxw = line::plane_threads(elem, std::max(x.r1, y.r1)) / 32, ncols = npol * g.nxc;
-    const int na = 32 / x.r2, nb = 32 / x.r1, nya = 32 / y.r2, nyb = 32 / y.r1;
-    const double ca = 2 * line::dft_ops(x.r1) + 10 * x.r1 + 40;
-    const double cb = npol * (2 * line::dft_ops(x.r2) + 12 * (x.r2 - 1) + 20 * x.r2);
-    const double cya = 2 * line::dft_ops(y.r1) + 30 * y.r1 + 40;
-    const double cyb = 2 * line::dft_ops(y.r2) + 12 * y.r2 + 20 * y.r2;
     std::vector<PlaneShape> all, out;
     for (int nw = 1; nw <= maxw; ++nw)
         for (int L = 1; L <= 12; ++L) {
             PlaneShape s;
             s.nw = nw;
             s.L = L;
-            s.smem = (size_t(ncols) * y.ld + size_t(nw) * npol * L * x.ld) * elem;
+            s.smem = (size_t(ncols) * y.ld + size_t(nw) * npol * L * x.ld) * elem + extra;
             if (s.smem > kSmemMax) break;
             s.ctas = std::min<int>({int(228 * 1024 / (s.smem + 1024)), maxw / nw, 32});
-            const int groups = ceil_div(ceil_div(y.n, L), nw), cper = ceil_div(ncols, nw);
-            s.work = groups * (ceil_div(npol * L, na) * ca + ceil_div(L, nb) * cb) + ceil_div(cper, nya) * cya +
-                     ceil_div(cper, nyb) * cyb;
+            s.work = warp_work(x, y, ncols, npol, nw, L, inverse_only);
             all.push_back(s);
         }
     std::stable_sort(all.begin(), all.end(), [](const PlaneShape& a, const PlaneShape& b) { return a.work < b.work; });
@@ -46,17 +52,24 @@ std::vector<PlaneShape> plane_shapes(const PWGrid& g, int prec, int npol) {
     return out;
 }
 
-// the shape for a launch of nctas planes: waves of resident CTAs times a CTA's time, which is its busiest warp's
-// (up to 16 warps of an SM run latency-bound, each at its own pace) plus a start-up of about 700 instructions
-const PlaneShape& pick_shape(const std::vector<PlaneShape>& c, long nctas) {
+// a CTA's time in instructions: its busiest warp's (up to 16 warps of an SM run latency-bound, each at its own pace)
+// plus a start-up of about 700
+constexpr double kStartUp = 700;
+long waves(long nctas, const PlaneShape& s) { return (nctas + long(kSMs) * s.ctas - 1) / (long(kSMs) * s.ctas); }
+
+// the shape for a launch of nctas planes, by waves of resident CTAs times a CTA's time; variant v > 1: the v-th best
+// by that estimate (the autotuner's candidates)
+const PlaneShape& pick_shape(const std::vector<PlaneShape>& c, long nctas, int variant) {
+    auto time_of = [&](const PlaneShape& s) { return double(waves(nctas, s)) * (s.work + kStartUp); };
     const PlaneShape* best = &c[0];
-    double bt = 1e300;
-    for (const PlaneShape& s : c) {
-        const double t = double((nctas + long(kSMs) * s.ctas - 1) / (long(kSMs) * s.ctas)) * (s.work + 700);
-        if (t < bt) {
-            bt = t;
-            best = &s;
-        }
+    double floor = -1;
+    for (int v = 0; v < std::max(1, variant); ++v) {
+        const PlaneShape* next = nullptr;
+        for (const PlaneShape& s : c)
+            if (time_of(s) > floor && (!next || time_of(s) < time_of(*next))) next = &s;
+        if (!next) break;  // fewer candidates than variants: the last one
+        best = next;
+        floor = time_of(*next);
     }
     return *best;
 }
@@ -69,7 +82,8 @@ int rmax_of(int r) { return r <= 10 ? 10 : r <= 16 ? 16 : 25; }
 template <typename T, typename R, int NPOL>
 void plane_pass(const PWGrid& g, int nplanes, const R* v, T* sb, cudaStream_t s) {
     constexpr int pi = sizeof(T) == 8;
-    const PlaneShape& sh = pick_shape(g.lines.shapes[pi][NPOL - 1], long(nplanes) * g.nz);
+    const PlaneShape& sh = pick_shape(g.lines.shapes[pi][NPOL - 1], long(nplanes) * g.nz,
+                                      pi ? g.plane_variant32 : g.plane_variant64);
     if constexpr (NPOL == 1)
         if (line::plane_fixed_a<T, R>(g, sh, nplanes, v, sb, s) || line::plane_fixed_b<T, R>(g, sh, nplanes, v, sb, s) ||
             line::plane_fixed_c<T, R>(g, sh, nplanes, v, sb, s))
@@ -165,7 +179,7 @@ void build_line_plan(PWGrid& g) {
         }
     }
     for (int i = 0; i < 2; ++i)
-        for (int npol = 1; npol <= 2; ++npol) p.shapes[i][npol - 1] = plane_shapes(g, i, npol);
+        for (int npol = 1; npol <= 2; ++npol) p.shapes[i][npol - 1] = plane_shapes(g, i, npol, false, 0);
     p.ok = true;
 }
 
@@ -210,13 +224,92 @@ bool launch_hpsi_local_nc_lines(const PWGrid& g, int ik, const R* veff4_zyx, int
     return true;
 }
 
+// ---- psi -> rho ----
+namespace {
+
+// rho[x][y][z] += sum over g < nsplit of ws[g][z][y][x] in a fixed order, a 32 x 32 tile of (x, z) per CTA
+template <typename R>
+__global__ void __launch_bounds__(256) k_rho_reduce(int nx, int ny, int nz, int nsplit, const R* __restrict__ ws,
+                                                    R* __restrict__ rho) {
+    __shared__ R tile[32][33];
+    const int x0 = blockIdx.x * 32, z0 = blockIdx.y * 32, y = blockIdx.z;
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const size_t N = size_t(nx) * ny * nz;
+    for (int r = ty; r < 32; r += 8) {
+        const int z = z0 + r, x = x0 + tx;
+        if (z >= nz || x >= nx) continue;
+        const R* p = ws + (size_t(z) * ny + y) * nx + x;
+        R sum = p[0];
+        for (int g = 1; g < nsplit; ++g) sum += p[size_t(g) * N];
+        tile[r][tx] = sum;
+    }
+    __syncthreads();
+    for (int r = ty; r < 32; r += 8) {
+        const int x = x0 + r, z = z0 + tx;
+        if (z < nz && x < nx) rho[(size_t(x) * ny + y) * nz + z] += tile[tx][r];
+    }
+}
+
+}  // namespace
+
+// the launch of psi -> rho for nbc bands: nsplit CTAs a plane share its bands, so that the planes of a small grid
+// fill the SMs; the partial planes take at most 512 MB
+RhoShape rho_shape(const PWGrid& g, size_t elem, int nbc) {
+    const int prec = elem == 8;
+    const size_t real = elem / 2, plane = size_t(g.nx) * g.ny * real;
+    RhoShape best;
+    double bt = 1e300;
+    for (const bool sums : {true, false}) {
+        for (const PlaneShape& s : plane_shapes(g, prec, 1, true, sums ? plane : 0))
+            for (int ns = 1; ns <= std::min(nbc, 64); ++ns) {
+                if (ns > 1 && size_t(ns) * g.nxyz() * real > size_t(512) << 20) break;
+                // sums kept in L2 cost about a quarter more than in shared memory; a partial plane is written and read
+                const double per_band = (s.work + kStartUp / 2) * (sums ? 1.0 : 1.25);
+                const double t = double(waves(long(g.nz) * ns, s)) * (ceil_div(nbc, ns) * per_band + kStartUp) +
+                                 0.02 * ns * double(g.nxyz()) / kSMs;
+                if (t < bt) {
+                    bt = t;
+                    best.plane = s;
+                    best.nsplit = ns;
+                    best.sums = sums;
+                }
+            }
+    }
+    return best;
+}
+
+template <typename T, typename R>
+void launch_rho_chunk(const PWGrid& g, const RhoShape& shape, int ik, int b0, int nbc, int ld, const T* psi,
+                      const double* w_chunk, T* sb, R* ws, int first, cudaStream_t s) {
+    constexpr int pi = sizeof(T) == 8;
+    const OneK src = one_k<T, R>(g, ik, ld, psi, nullptr);
+    z_pass<T, R>(true, g, src, 1, b0, nbc, sb, 0.0, 0, s);
+    const line::RhoArgs<T, R> a{shape, sb, nbc, w_chunk, ws, first, s};
+    if (line::rho_fixed<T, R>(g, a)) return;
+    const LineGeom &x = g.lines.x[pi], &y = g.lines.y[pi];
+    switch (rmax_of(std::max(x.r1, y.r1))) {
+        case 10: line::rho_launch<T, R, 10>(g, x, y, a); break;
+        case 16: line::rho_launch<T, R, 16>(g, x, y, a); break;
+        default: line::rho_launch<T, R, 25>(g, x, y, a); break;
+    }
+}
+
+template <typename R> void launch_rho_reduce(const PWGrid& g, int nsplit, const R* ws, R* rho, cudaStream_t s) {
+    k_rho_reduce<R><<<dim3(ceil_div(g.nx, 32), ceil_div(g.nz, 32), g.ny), 256, 0, s>>>(g.nx, g.ny, g.nz, nsplit, ws, rho);
+    note_launch();
+    B200_CUDA(cudaGetLastError());
+}
+
 #define B200_INST(T, R)                                                                                              \
     template bool launch_hpsi_local_lines<T, R>(const PWGrid&, int, const R*, int, int, const T*, T*, T*, double, int, \
                                                 cudaStream_t);                                                       \
     template bool launch_hpsi_local_kbatch_lines<T, R>(const PWGrid&, const KBatchArgs&, int, int, const R*, T*, int,  \
                                                        double, cudaStream_t);                                        \
     template bool launch_hpsi_local_nc_lines<T, R>(const PWGrid&, int, const R*, int, int, const T*, T*, T*, double,   \
-                                                   cudaStream_t);
+                                                   cudaStream_t);                                                    \
+    template void launch_rho_chunk<T, R>(const PWGrid&, const RhoShape&, int, int, int, int, const T*, const double*,  \
+                                         T*, R*, int, cudaStream_t);                                                 \
+    template void launch_rho_reduce<R>(const PWGrid&, int, const R*, R*, cudaStream_t);
 B200_INST(double2, double)
 B200_INST(float2, float)
 #undef B200_INST

@@ -111,24 +111,12 @@ void Hamilt::set_veff(const double* veff_d) {
     launch_transpose_veff<double>(*grid, veff_d, veff_zyx.ptr, 0);
     veff_zyxf.resize(N);
     launch_transpose_veff<float>(*grid, veff_d, veff_zyxf.ptr, 0);
-    has_perm = plane_perm_supported(*grid);
-    if (has_perm) {
-        // two layouts back to back: the warp-shuffle plane pass's, then the two-pass plane pass's
-        veff_perm.resize(2 * N);
-        veff_permf.resize(2 * N);
-        launch_permute_veff<double>(*grid, veff_zyx.ptr, veff_perm.ptr, 0);
-        launch_permute_veff<float>(*grid, veff_zyxf.ptr, veff_permf.ptr, 0);
-        launch_arrange_veff<double>(*grid, veff_zyx.ptr, veff_perm.ptr + N, 0);
-        launch_arrange_veff<float>(*grid, veff_zyxf.ptr, veff_permf.ptr + N, 0);
-    }
     B200_CUDA(cudaStreamSynchronize(0));
     has_veff = true;
 }
 
 template <> const double* Hamilt::veff_of<double>() const { return veff_zyx.ptr; }
 template <> const float* Hamilt::veff_of<float>() const { return veff_zyxf.ptr; }
-template <> const double* Hamilt::veff_perm_of<double>() const { return has_perm ? veff_perm.ptr : nullptr; }
-template <> const float* Hamilt::veff_perm_of<float>() const { return has_perm ? veff_permf.ptr : nullptr; }
 
 void Hamilt::set_vkb(int ik, int nkb, int npwx, const double2* vkb_d) {
     B200_CHECK(ik >= 0 && ik < int(nl.size()), kInvalidArgument, "k-point index out of range");
@@ -291,11 +279,10 @@ void Hamilt::set_fp64_gemm(int mode, int nmods) {
     B200_CUDA(cudaStreamSynchronize(0));
 }
 
-int Hamilt::band_chunk(size_t elem) const {
+int Hamilt::band_chunk(size_t elem, size_t stick_bytes) const {
     if (chunk_override > 0) return chunk_override;
-    // keep one chunk's stick buffer (nst*nz per band) inside ~48 MB so the three passes hit L2
     const size_t per_band = size_t(grid->nst) * grid->nz * elem;
-    size_t c = (size_t(48) << 20) / (per_band ? per_band : 1);
+    size_t c = stick_bytes / (per_band ? per_band : 1);
     if (c < 1) c = 1;
     if (c > 4096) c = 4096;
     return int(c);
@@ -335,7 +322,7 @@ void Hamilt::hpsi(int ik, int spin, int nb, int ld, const T* psi, T* hpsi, int m
     auto local_pass = [&](cudaStream_t st) {
         B200_CHECK(has_veff, kInvalidArgument, "V_eff not set");
         const R* veff = f64 ? (const R*)veff_zyx.ptr : (const R*)veff_zyxf.ptr;
-        const int chunk = band_chunk(sizeof(T));
+        const int chunk = band_chunk(sizeof(T), W.stick_bytes);
         const int nbc0 = nb < chunk ? nb : chunk;
         const size_t sbn = size_t(nbc0) * grid->nst * grid->nz;
         T* sb;
@@ -348,7 +335,7 @@ void Hamilt::hpsi(int ik, int spin, int nb, int ld, const T* psi, T* hpsi, int m
         }
         for (int b0 = 0; b0 < nb; b0 += chunk) {
             const int nbc = nb - b0 < chunk ? nb - b0 : chunk;
-            launch_hpsi_local<T, R>(*grid, ik, veff, veff_perm_of<R>(), nbc, ld, psi + size_t(b0) * ld,
+            launch_hpsi_local<T, R>(*grid, ik, veff, nbc, ld, psi + size_t(b0) * ld,
                                     hpsi + size_t(b0) * ld, sb, grid->basis.tpiba2, 0, st);
         }
     };
@@ -542,7 +529,7 @@ void Hamilt::hpsi_kbatch(int nk, const int* iks, int spin, int nb, int ld, const
         args.e[q].gk2 = f64 ? (const void*)km.gk2.ptr : (const void*)km.gk2f.ptr;
     }
     const size_t per_band = size_t(grid->nst) * grid->nz * sizeof(T);
-    int chunk = chunk_override > 0 ? chunk_override : int((size_t(48) << 20) / (per_band * nk));
+    int chunk = chunk_override > 0 ? chunk_override : int(std::min<size_t>(nb, W.stick_bytes / (per_band * nk)));
     if (chunk < 1) chunk = 1;
     if (chunk > nb) chunk = nb;
     const R* veff = f64 ? (const R*)veff_zyx.ptr : (const R*)veff_zyxf.ptr;
@@ -554,8 +541,7 @@ void Hamilt::hpsi_kbatch(int nk, const int* iks, int spin, int nb, int ld, const
         W.sb32.resize(size_t(nk) * chunk * grid->nst * grid->nz);
         sb = W.sb32.ptr;
     }
-    if (!launch_hpsi_local_kbatch<T, R>(*grid, args, nk, nb, veff, veff_perm_of<R>(), sb, chunk, grid->basis.tpiba2,
-                                        s)) {
+    if (!launch_hpsi_local_kbatch_lines<T, R>(*grid, args, nk, nb, veff, sb, chunk, grid->basis.tpiba2, s)) {
         for (int q = 0; q < nk; ++q) hpsi<T>(iks[q], spin, nb, ld, psis[q], hpsis[q], 1, s, &W);
     }
     for (int q = 0; q < nk; ++q) hpsi<T>(iks[q], spin, nb, ld, psis[q], hpsis[q], 2, s, &W);

@@ -42,6 +42,7 @@ struct NonlocalK {
 // tensor-core GEMM workspace.  Callers that run H|psi> concurrently (different streams or threads) each
 // own one; the Hamiltonian itself is read-only after set-up.
 struct HpsiWork {
+    size_t stick_bytes = kStickBytes;  // limit of a band chunk's stick buffer
     DeviceArray<double2> sb64, becp64, rb64;
     DeviceArray<float2> sb32, becp32, psi_pad32, rb32;  // rb: real-space planes of the npol = 2 local pass
     cublasHandle_t cublas = nullptr;
@@ -81,13 +82,7 @@ struct Hamilt {
     int precision = 0;  // 0 = FP64, 1 = mixed
     DeviceArray<double> veff_zyx;
     DeviceArray<float> veff_zyxf;
-    // grids with 32*m square planes: (z, y, x) in the warp-shuffle register-transform order, then (N more
-    // values) the arrangement of the two-pass plane transforms
-    DeviceArray<double> veff_perm;
-    DeviceArray<float> veff_permf;
-    bool has_perm = false;
     template <typename R> const R* veff_of() const;
-    template <typename R> const R* veff_perm_of() const;
     bool has_veff = false;
     std::vector<NonlocalK> nl;
     int ntype = 0, nspin = 1, dx = 0, dy = 0, dz = 0;
@@ -101,7 +96,7 @@ struct Hamilt {
     DeviceArray<double2> deeq_nc;
     int nc_dx = 0, nc_dy = 0, nc_dz = 0;
     HpsiWork work;  // default scratch for callers that do not bring their own
-    int chunk_override = 0;  // bands per stick-buffer chunk chosen by the autotuner (0 = 48 MB rule)
+    int chunk_override = 0;  // bands per stick-buffer chunk chosen by the autotuner (0 = the scratch's stick_bytes)
     // FP64 projector products: 0 = cuBLAS ZGEMM; int8 tensor cores (exact modular emulation, oz_mods moduli)
     // 1 = for calls of at least kOzMinBands bands (each call reads the projectors' whole residue form, twice the
     // bytes of the FP64 projectors, so narrow calls go to cuBLAS, whose cost scales with the bands), 2 = always
@@ -122,7 +117,7 @@ struct Hamilt {
     void set_veff(const double* veff_d);
     void set_vkb(int ik, int nkb, int npwx, const double2* vkb_d);
     void set_deeq(int ntype, const int* na, const int* nh, int nspin, int dx, int dy, int dz, const double* deeq_d);
-    int band_chunk(size_t elem) const;
+    int band_chunk(size_t elem, size_t stick_bytes) const;
     // fold D into the projectors of k-point ik (all spins), on stream s; nothing if either is not set.  With
     // fp64_gemm = 1 also the int8 residue forms of vkb and vkbd.
     void fold_projectors(int ik, cudaStream_t s);

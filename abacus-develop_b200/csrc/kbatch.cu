@@ -100,9 +100,9 @@ int b200_hamilt_autotune(b200_hamilt* h, int ik, int nbands, int ld, const void*
         cand.push_back(nbands);
         std::sort(cand.begin(), cand.end());
         cand.erase(std::unique(cand.begin(), cand.end()), cand.end());
-        // plane-pass variants: only grids with the register transforms have a choice
+        // launch shapes of the plane pass: only grids with the line transforms have a choice
         std::vector<int> vars = {variant};
-        if (b200::plane_perm_supported(G)) {
+        if (b200::lines_supported(G, f64 ? 16 : 8, 1)) {
             vars.clear();
             for (int v = 1; v <= b200::kPlaneVariants; ++v) vars.push_back(v);
         }

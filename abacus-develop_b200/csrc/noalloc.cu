@@ -77,10 +77,9 @@ void hpsi_local_noalloc(b200::Hamilt& H, int ik, int nb, int ld, const T* psi, T
     // bands per launch: what the scratch holds, and at most 65535 (the launches put bands on gridDim.y)
     const int chunk = int(std::min<size_t>(kNoAllocScratchBytes / per_band, 65535));
     const R* veff = H.veff_of<R>();
-    const R* veffp = H.veff_perm_of<R>();
     for (int b0 = 0; b0 < nb; b0 += chunk) {
         const int nbc = nb - b0 < chunk ? nb - b0 : chunk;
-        b200::launch_hpsi_local<T, R>(g, ik, veff, veffp, nbc, ld, psi + size_t(b0) * ld, hpsi + size_t(b0) * ld, sb,
+        b200::launch_hpsi_local<T, R>(g, ik, veff, nbc, ld, psi + size_t(b0) * ld, hpsi + size_t(b0) * ld, sb,
                                       g.basis.tpiba2, 0, s);
     }
 }

@@ -33,6 +33,78 @@ namespace line {
 
 template <typename T> __device__ __forceinline__ T zero_of() { return cmake<T>(0, 0); }
 
+// inverse y transform of the columns [c0, c1) of a warp: pass A straight from the sticks, pass B in place
+template <typename T, int RMAX, int NPOL, typename GY, typename Tw>
+__device__ __forceinline__ void inverse_y(const PlaneMapView& pm, const GY& gy, int lane, int c0, int c1,
+                                          const T* __restrict__ plane, size_t pcomp, T* A, const Tw& twy) {
+    const int nxc = pm.nxc;
+    const int la = lane / gy.r2, ta = lane - la * gy.r2, na = 32 / gy.r2;
+    for (int c = c0 + la; c < c1; c += na) {
+        if (la >= na) break;
+        const int cc = NPOL == 1 ? c : (c >= nxc ? c - nxc : c);
+        const int4 d = __ldg(pm.cd + cc);
+        const T* src = plane + (NPOL == 2 && c >= nxc ? pcomp : 0) + d.x;
+        T* col = A + c * gy.ld + ta;
+        with_r1<RMAX>(gy, [&](auto q) {
+            constexpr int Q = decltype(q)::value;
+            T u[Q];
+#pragma unroll
+            for (int n1 = 0; n1 < Q; ++n1) {
+                const int y = n1 * gy.r2 + ta;
+                const bool lo = y < d.y, hi = y >= d.z && y < d.w;
+                u[n1] = (lo || hi) ? src[lo ? y : d.y + y - d.z] : zero_of<T>();
+            }
+            dft<T, +1, Q>(u);
+#pragma unroll
+            for (int k1 = 0; k1 < Q; ++k1) col[k1 * gy.rs] = u[k1];
+        });
+    }
+    __syncwarp();
+    const int lb = lane / gy.r1, k1 = lane - lb * gy.r1, nb = 32 / gy.r1;
+    for (int c = c0 + lb; c < c1; c += nb) {
+        if (lb >= nb) break;
+        T* blk = A + c * gy.ld + k1 * gy.rs;
+        with_r2<RMAX>(gy, [&](auto q) {
+            constexpr int Q = decltype(q)::value;
+            T w[Q];
+            w[0] = blk[0];
+#pragma unroll
+            for (int t = 1; t < Q; ++t) w[t] = cmulc(blk[t], twy(t, k1));
+            dft<T, +1, Q>(w);
+#pragma unroll
+            for (int k2 = 0; k2 < Q; ++k2) blk[k2] = w[k2];
+        });
+    }
+}
+// inverse x transform, pass A, of rows [y0, y0 + nl) (of each component) into the row buffer
+template <typename T, int RMAX, int NPOL, typename GX, typename GY>
+__device__ __forceinline__ void inverse_x_rows(const PlaneMapView& pm, const GX& gx, const GY& gy, int lane, int y0, int nl,
+                                               const T* A, T* buf) {
+    const int nxc = pm.nxc;
+    const int la = lane / gx.r2, ta = lane - la * gx.r2, na = 32 / gx.r2;
+    for (int l = la; l < NPOL * nl; l += na) {
+        if (la >= na) break;
+        const int lr = NPOL == 1 ? l : (l >= nl ? l - nl : l);
+        const int y = y0 + lr;
+        const int yq = y / gy.r1;
+        const T* row = A + (y - yq * gy.r1) * gy.rs + yq + (NPOL == 2 && l >= nl ? nxc * gy.ld : 0);
+        T* b = buf + l * gx.ld + ta;
+        with_r1<RMAX>(gx, [&](auto q) {
+            constexpr int Q = decltype(q)::value;
+            T u[Q];
+#pragma unroll
+            for (int n1 = 0; n1 < Q; ++n1) {
+                const int x = n1 * gx.r2 + ta;
+                const bool lo = x < pm.xm, hi = x >= pm.xh;
+                u[n1] = (lo || hi) ? row[(lo ? x : x - pm.xoff) * gy.ld] : zero_of<T>();
+            }
+            dft<T, +1, Q>(u);
+#pragma unroll
+            for (int j = 0; j < Q; ++j) b[j * gx.rs] = u[j];
+        });
+    }
+}
+
 // ---- plane pass ----
 // NPOL = 1: v = V_eff (z, y, x).  NPOL = 2: columns 2b and 2b + 1 of the stick buffer are the components of band
 // b = blockIdx.x, v the four components of V_eff (pitch vstride), applied as veff_pw_op's 2 x 2 form.
@@ -64,46 +136,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_plane_g(PlaneMapView pm, GX gx, GY 
         if constexpr (kSame) return tw[t];
         else return __ldg(rooty + t * k1);
     };
-    {
-        const int la = lane / gy.r2, ta = lane - la * gy.r2, na = 32 / gy.r2;
-        // inverse y, pass A: straight from the sticks
-        for (int c = c0 + la; c < c1; c += na) {
-            if (la >= na) break;
-            const int cc = NPOL == 1 ? c : (c >= nxc ? c - nxc : c);
-            const int4 d = __ldg(pm.cd + cc);
-            const T* src = plane + (NPOL == 2 && c >= nxc ? pcomp : 0) + d.x;
-            T* col = A + c * gy.ld + ta;
-            with_r1<RMAX>(gy, [&](auto q) {
-                constexpr int Q = decltype(q)::value;
-                T u[Q];
-#pragma unroll
-                for (int n1 = 0; n1 < Q; ++n1) {
-                    const int y = n1 * gy.r2 + ta;
-                    const bool lo = y < d.y, hi = y >= d.z && y < d.w;
-                    u[n1] = (lo || hi) ? src[lo ? y : d.y + y - d.z] : zero_of<T>();
-                }
-                dft<T, +1, Q>(u);
-#pragma unroll
-                for (int k1 = 0; k1 < Q; ++k1) col[k1 * gy.rs] = u[k1];
-            });
-        }
-        __syncwarp();
-        const int lb = lane / gy.r1, k1 = lane - lb * gy.r1, nb = 32 / gy.r1;
-        for (int c = c0 + lb; c < c1; c += nb) {
-            if (lb >= nb) break;
-            T* blk = A + c * gy.ld + k1 * gy.rs;
-            with_r2<RMAX>(gy, [&](auto q) {
-                constexpr int Q = decltype(q)::value;
-                T w[Q];
-                w[0] = blk[0];
-#pragma unroll
-                for (int t = 1; t < Q; ++t) w[t] = cmulc(blk[t], twy(t, k1));
-                dft<T, +1, Q>(w);
-#pragma unroll
-                for (int k2 = 0; k2 < Q; ++k2) blk[k2] = w[k2];
-            });
-        }
-    }
+    inverse_y<T, RMAX, NPOL>(pm, gy, lane, c0, c1, plane, pcomp, A, twy);
     __syncthreads();
     // ---- rows: inverse x, V_eff, forward x ----
     {
@@ -121,27 +154,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_plane_g(PlaneMapView pm, GX gx, GY 
         for (int y0 = warp * L; y0 < gy.n; y0 += nw * L) {
             const int nl = min(L, gy.n - y0);
             if (NPOL == 1 && lb < nb && lb < nl) load_v(y0 + lb);
-            for (int l = la; l < NPOL * nl; l += na) {
-                if (la >= na) break;
-                const int lr = NPOL == 1 ? l : (l >= nl ? l - nl : l);
-                const int y = y0 + lr;
-                const int yq = y / gy.r1;
-                const T* row = A + (y - yq * gy.r1) * gy.rs + yq + (NPOL == 2 && l >= nl ? nxc * gy.ld : 0);
-                T* b = buf + l * gx.ld + ta;
-                with_r1<RMAX>(gx, [&](auto q) {
-                    constexpr int Q = decltype(q)::value;
-                    T u[Q];
-#pragma unroll
-                    for (int n1 = 0; n1 < Q; ++n1) {
-                        const int x = n1 * gx.r2 + ta;
-                        const bool lo = x < pm.xm, hi = x >= pm.xh;
-                        u[n1] = (lo || hi) ? row[(lo ? x : x - pm.xoff) * gy.ld] : zero_of<T>();
-                    }
-                    dft<T, +1, Q>(u);
-#pragma unroll
-                    for (int j = 0; j < Q; ++j) b[j * gx.rs] = u[j];
-                });
-            }
+            inverse_x_rows<T, RMAX, NPOL>(pm, gx, gy, lane, y0, nl, A, buf);
             __syncwarp();
             for (int l = lb; l < nl; l += nb) {
                 if (lb >= nb) break;
@@ -262,6 +275,75 @@ __global__ void __launch_bounds__(MAXT, 1) k_plane_g(PlaneMapView pm, GX gx, GY 
                 }
             });
         }
+    }
+}
+
+// ---- psi -> rho: w_b |psi_b(r)|^2 summed over bands g, g + nsplit, ... of the stick buffer, at plane z ----
+// One CTA per (z, g = blockIdx.y).  The sums of a CTA's plane live in shared memory after the row buffers, or, where
+// that does not fit (sums = false), in its own plane of ws (in L2).  A point is always added to by the same thread,
+// so nothing orders the sums but the band loop, and they are deterministic.  ws[g] is overwritten on the first chunk
+// of bands and added to afterwards.
+template <typename T, typename R, int RMAX, int MAXT, typename GX, typename GY>
+__global__ void __launch_bounds__(MAXT, 1) k_rho_g(PlaneMapView pm, GX gx, GY gy, int L, int nz,
+                                                   const T* __restrict__ rootx, const T* __restrict__ rooty,
+                                                   const T* __restrict__ sb, int nbc, const double* __restrict__ w,
+                                                   int nsplit, bool sums, R* __restrict__ ws, int first) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    T* A = reinterpret_cast<T*>(smem_raw);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int nxc = pm.nxc, z = blockIdx.x, g = blockIdx.y;
+    const size_t plane_n = size_t(gy.n) * gx.n;
+    R* out = ws + (size_t(g) * nz + z) * plane_n;
+    R* acc = sums ? reinterpret_cast<R*>(A + nxc * gy.ld + nw * L * gx.ld) : out;
+    const int cper = (nxc + nw - 1) / nw;
+    const int c0 = warp * cper, c1 = min(nxc, c0 + cper);
+    constexpr int kTw = MaxR2<GX>::value;
+    constexpr bool kSame = SameLine<GX, GY>::value;
+    const int lb = lane / gx.r1, k1 = lane - lb * gx.r1, nb = 32 / gx.r1;
+    T tw[kTw];
+#pragma unroll
+    for (int t = 1; t < kTw; ++t) tw[t] = t < gx.r2 ? __ldg(rootx + t * k1) : zero_of<T>();
+    auto twy = [&](int t, int ky) {
+        if constexpr (kSame) return tw[t];
+        else return __ldg(rooty + t * ky);
+    };
+    T* buf = A + nxc * gy.ld + warp * L * gx.ld;
+    for (int b = g; b < nbc; b += nsplit) {
+        const R wb = R(w[b]);
+        const bool init = b == g && (sums || first);
+        inverse_y<T, RMAX, 1>(pm, gy, lane, c0, c1, sb + (size_t(b) * nz + z) * pm.nst, 0, A, twy);
+        __syncthreads();
+        for (int y0 = warp * L; y0 < gy.n; y0 += nw * L) {
+            const int nl = min(L, gy.n - y0);
+            inverse_x_rows<T, RMAX, 1>(pm, gx, gy, lane, y0, nl, A, buf);
+            __syncwarp();
+            for (int l = lb; l < nl; l += nb) {
+                if (lb >= nb) break;
+                const T* bl = buf + l * gx.ld + k1 * gx.rs;
+                R* a = acc + size_t(y0 + l) * gx.n + k1;
+                with_r2<RMAX>(gx, [&](auto q) {
+                    constexpr int Q = decltype(q)::value;
+                    T v[Q];
+                    v[0] = bl[0];
+#pragma unroll
+                    for (int t = 1; t < Q; ++t) v[t] = cmulc(bl[t], tw[t]);
+                    dft<T, +1, Q>(v);
+#pragma unroll
+                    for (int k2 = 0; k2 < Q; ++k2) {
+                        const R n2 = fma(v[k2].x, v[k2].x, v[k2].y * v[k2].y);
+                        a[k2 * gx.r1] = init ? wb * n2 : fma(wb, n2, a[k2 * gx.r1]);
+                    }
+                });
+            }
+            __syncwarp();
+        }
+        __syncthreads();  // the columns are read
+    }
+    if (g >= nbc) {
+        if (first)
+            for (size_t i = threadIdx.x; i < plane_n; i += blockDim.x) out[i] = R(0);
+    } else if (sums) {
+        for (size_t i = threadIdx.x; i < plane_n; i += blockDim.x) out[i] = first ? acc[i] : out[i] + acc[i];
     }
 }
 

@@ -49,6 +49,36 @@ bool plane_fixed(const PWGrid& g, const PlaneShape& sh, int nplanes, const R* v,
     return true;
 }
 
+// launch of psi -> rho for the bands of one stick-buffer chunk (shape: rho_shape)
+template <typename T, typename R> struct RhoArgs {
+    const RhoShape& shape;
+    const T* sb;
+    int nbc;
+    const double* w;
+    R* ws;
+    int first;
+    cudaStream_t s;
+};
+template <typename T, typename R, int RMAX, typename GX, typename GY>
+void rho_launch(const PWGrid& g, GX gx, GY gy, const RhoArgs<T, R>& a) {
+    auto kern = k_rho_g<T, R, RMAX, plane_threads(sizeof(T), RMAX), GX, GY>;
+    const PlaneShape& sh = a.shape.plane;
+    set_smem(kern, sh.smem);
+    kern<<<dim3(g.nz, a.shape.nsplit), sh.nw * 32, sh.smem, a.s>>>(g.plane_view(), gx, gy, sh.L, g.nz, roots_of<T>(g.ax),
+                                                                  roots_of<T>(g.ay), a.sb, a.nbc, a.w, a.shape.nsplit,
+                                                                  a.shape.sums, a.ws, a.first);
+    note_launch();
+    B200_CUDA(cudaGetLastError());
+}
+template <typename T, typename R, int N> bool rho_fixed_n(const PWGrid& g, const RhoArgs<T, R>& a) {
+    constexpr int elem = sizeof(T);
+    constexpr LineGeom x = x_geom(N, elem), y = y_geom(N, elem, x.r2);
+    rho_launch<T, R, x.r1>(g, FixedGeom<N, x.r1, x.r2, x.rs, x.ld>(), FixedGeom<N, y.r1, y.r2, y.rs, y.ld>(), a);
+    return true;
+}
+// square planes with compiled lines; false for other grids (rho_f64.cu, rho_f32.cu)
+template <typename T, typename R> bool rho_fixed(const PWGrid& g, const RhoArgs<T, R>& a);
+
 // the z passes take one k-point (OneK) or a batch indexed by blockIdx.z (ManyK)
 struct OneK {
     KBatchEntry e;

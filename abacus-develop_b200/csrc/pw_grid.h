@@ -28,7 +28,7 @@ struct FftAxis {
     std::vector<double2> h_tw64;
     DeviceArray<double2> tw64;
     DeviceArray<float2> tw32;
-    DeviceArray<double2> rt64;  // the n roots W_n^j = exp(-2 pi i j / n), j < n (register/shuffle transforms)
+    DeviceArray<double2> rt64;  // the n roots W_n^j = exp(-2 pi i j / n), j < n (line transforms)
     DeviceArray<float2> rt32;
     void build(int n);  // host plan + twiddles
     void upload();
@@ -99,7 +99,7 @@ struct PWGrid {
     std::vector<int4> h_cdesc;
     DeviceArray<int4> cdesc;
     bool on_device = false;
-    // plane pass of the register transforms, per precision (0: default shape; see plane_launch_var)
+    // launch shape of the plane pass on the line transforms, per precision (0, 1: the estimate's best, v: its v-th)
     int plane_variant64 = 0, plane_variant32 = 0;
 
     void build(const PWBasisK& b);  // host-side plans and maps only (no GPU needed)
@@ -127,13 +127,8 @@ size_t plane_smem(const PWGrid& g, size_t elem);
 // ---- launchers (fft_kernels.cu); all asynchronous on `s` ----
 // Fused local part of H|psi> for nb bands (one chunk): hpsi = Ekin psi + V_loc psi (accumulate==0 zeroes padding).
 template <typename T, typename R>
-void launch_hpsi_local(const PWGrid& g, int ik, const R* veff_zyx, const R* veff_perm, int nb, int ld, const T* psi,
+void launch_hpsi_local(const PWGrid& g, int ik, const R* veff_zyx, int nb, int ld, const T* psi,
                        T* hpsi, T* stickbuf, double tpiba2, int accumulate, cudaStream_t s);
-// Same, on the register transforms of the 64-, 96- and 128-point grids; returns false (launching nothing) for
-// other grids.
-template <typename T, typename R>
-bool launch_hpsi_local_fast(const PWGrid& g, int ik, const R* veff_perm, int nb, int ld, const T* psi, T* hpsi,
-                            T* stickbuf, double tpiba2, int accumulate, cudaStream_t s);
 // k-point batch: one entry per k (its stick maps, psi / hpsi with leading dimension ld, npwk, gk2 in the
 // precision of the call); passed by value so a launch needs no device-side argument buffer.
 constexpr int kMaxKBatch = 128;
@@ -147,11 +142,6 @@ struct KBatchEntry {
 struct KBatchArgs {
     KBatchEntry e[kMaxKBatch];
 };
-// Kinetic + local part of H|psi> for nb bands of nk k-points in one launch per pass (per band chunk);
-// returns false for grid sizes without compiled warp transforms.
-template <typename T, typename R>
-bool launch_hpsi_local_kbatch(const PWGrid& g, const KBatchArgs& args, int nk, int nb, const R* veff_zyx,
-                              const R* veff_perm, T* stickbuf, int chunk, double tpiba2, cudaStream_t s);
 // The line transforms of grid g (host; fills g.lines and the run descriptors of columns and sticks).
 void build_line_plan(PWGrid& g);
 // The three passes on the line transforms (fft_lines.cu); false (nothing launched) where g.lines does not hold or a
@@ -180,26 +170,24 @@ void launch_real_to_recip(const PWGrid& g, int ik, const T* in, T* out, T* aux, 
 // V_eff (ABACUS r order) -> (z, y, x) transposed copy, in precision R.
 template <typename R>
 void launch_transpose_veff(const PWGrid& g, const double* veff, R* out, cudaStream_t s);
-// Square xy planes of n = 32*m (m = 2, 3, 4) use register/shuffle transforms whose r-space values come out
-// in a permuted order; V_eff is stored once in that order: out[z][sy][sx] = veff_zyx[z][p(sy)][p(sx)],
-// p(s) = s/32 + m*bitrev5(s mod 32).  Returns false (nothing done) for other grids.
-bool plane_perm_supported(const PWGrid& g);
-// psi -> rho on the register transforms (grids with plane_perm_supported whose plane fits shared memory):
-// bands [b0, b0 + nbc) of psi through the inverse z pass into sb, then w_chunk[b] |psi_b(r)|^2 summed into
-// nsplit partial planes ws (slot order; first = 1 overwrites them); launch_rho_reduce_r adds them to rho
-bool rho_r_supported(const PWGrid& g);
+// psi -> rho on the line transforms (where lines_supported): rho_shape chooses the launch for chunks of up to nbc
+// bands; bands [b0, b0 + nbc) of psi go through the inverse z pass into sb, then w_chunk[b] |psi_b(r)|^2 is summed into
+// shape.nsplit partial grids ws in (z, y, x) order (first = 1 overwrites them); launch_rho_reduce adds them to rho
+struct RhoShape {
+    PlaneShape plane;
+    int nsplit = 0;
+    bool sums = false;  // a CTA's sums in shared memory
+};
+RhoShape rho_shape(const PWGrid& g, size_t elem, int nbc);
 template <typename T, typename R>
-void launch_rho_chunk_r(const PWGrid& g, int ik, int b0, int nbc, int ld, const T* psi, const double* w_chunk,
-                        T* sb, int nsplit, R* ws, int first, cudaStream_t s);
-template <typename R>
-void launch_rho_reduce_r(const PWGrid& g, int nsplit, const R* ws, R* rho, cudaStream_t s);
-template <typename R>
-bool launch_permute_veff(const PWGrid& g, const R* veff_zyx, R* out, cudaStream_t s);
-// The same grids: V_eff arranged for the two-pass plane transforms, out[z slot][p][k1][k2] =
-// veff_zyx[z][y(p)][k1 + R1 k2] with N = 8 R1, y(p) = p/8 + R1 (p mod 8) (plane_t.cuh)
-template <typename R>
-bool launch_arrange_veff(const PWGrid& g, const R* veff_zyx, R* out, cudaStream_t s);
-// Number of plane-pass variants the autotuner may choose from (1 .. kPlaneVariants)
+void launch_rho_chunk(const PWGrid& g, const RhoShape& shape, int ik, int b0, int nbc, int ld, const T* psi,
+                      const double* w_chunk, T* sb, R* ws, int first, cudaStream_t s);
+template <typename R> void launch_rho_reduce(const PWGrid& g, int nsplit, const R* ws, R* rho, cudaStream_t s);
+// Stick buffer of a band chunk of the local passes.  One launch over many bands has fewer partly filled waves: 160
+// bands at 96^3 in FP64 run 1.35 ms in one chunk of 428 MB, 1.47 ms in chunks of 48 MB (which do not stay in L2
+// either way), 480 bands at 128^3 in FP32 5.27 ms at 512 MB, 5.20 at 1.6 GB, 5.68 at 48 MB.
+constexpr size_t kStickBytes = size_t(512) << 20;
+// Number of plane-pass launch shapes the autotuner may choose from (1 .. kPlaneVariants)
 constexpr int kPlaneVariants = 5;
 
 }  // namespace b200

@@ -3,9 +3,9 @@
 //
 // The functor entry points mirror the reference (rho is an array of nspin device pointers, host side).  The
 // product path b200_pw_basis_psi_to_rho computes the reference's sum rho(r) += w1_b |psi_b(r)|^2 over the
-// bands with a non-zero weight: on grids with register transforms (nx = ny and nx, nz in {64, 96, 128})
+// bands with a non-zero weight: on grids with line transforms (plane_g.cuh)
 // fused into two passes per band chunk (inverse z transform of the sticks; per z plane the inverse y and x
-// transforms with |psi|^2 summed in registers) and one final reduction; elsewhere by the reference's loop,
+// transforms with |psi|^2 summed by the same CTA) and one final reduction; elsewhere by the reference's loop,
 // the drop-in transform recip_to_real into a full box and elecstate_pw_op per band.  Nothing goes back to
 // the host between bands.  One call at a time per basis handle (its scratch is shared).
 #include <algorithm>
@@ -94,16 +94,16 @@ void psi_to_rho(b200_pw_basis* b, b200::DeviceArray<T>& box, b200::DeviceArray<T
     B200_CHECK(nbands >= 0 && ld >= g.kmaps[ik].npw, b200::kInvalidArgument, "ld smaller than npwk");
     B200_CHECK(psi && w1 && rho, b200::kInvalidArgument, "NULL argument");
     g.ensure_device();
-    if (nbands > 0 && b200::rho_r_supported(g)) {
-        // the same sum on the register transforms: runs of consecutive bands with a non-zero weight (the
-        // reference skips the others, elecstate_pw.cpp:211), in chunks whose stick buffer is about 48 MB
+    if (nbands > 0 && b200::lines_supported(g, sizeof(T), 1)) {
+        // the same sum on the line transforms: runs of consecutive bands with a non-zero weight (the
+        // reference skips the others, elecstate_pw.cpp:211), in chunks whose stick buffer is at most kStickBytes
         b->rho_w.resize(size_t(nbands));
         B200_CUDA(cudaMemcpyAsync(b->rho_w.ptr, w1, size_t(nbands) * sizeof(double), cudaMemcpyHostToDevice, s));
         const size_t per_band = size_t(g.nz) * g.nst;
-        const int chunk = int(std::max<size_t>(1, (size_t(48) << 20) / (per_band * sizeof(T))));
-        sbuf.resize(size_t(std::min(chunk, nbands)) * per_band);
-        const int nsplit = std::max(1, std::min(8, (2 * 148 + g.nz - 1) / g.nz));  // about two CTAs per SM
-        ws.resize(size_t(nsplit) * size_t(g.nxyz()));
+        const int chunk = int(std::min<size_t>(nbands, std::max<size_t>(1, b200::kStickBytes / (per_band * sizeof(T)))));
+        sbuf.resize(size_t(chunk) * per_band);
+        const b200::RhoShape shape = b200::rho_shape(g, sizeof(T), chunk);
+        ws.resize(size_t(shape.nsplit) * size_t(g.nxyz()));
         int first = 1;
         for (int b0 = 0; b0 < nbands;) {
             if (w1[b0] == 0.0) {
@@ -112,12 +112,11 @@ void psi_to_rho(b200_pw_basis* b, b200::DeviceArray<T>& box, b200::DeviceArray<T
             }
             int b1 = b0;
             while (b1 < nbands && w1[b1] != 0.0 && b1 - b0 < chunk) ++b1;
-            b200::launch_rho_chunk_r<T, R>(g, ik, b0, b1 - b0, ld, psi, b->rho_w.ptr + b0, sbuf.ptr, nsplit, ws.ptr,
-                                           first, s);
+            b200::launch_rho_chunk<T, R>(g, shape, ik, b0, b1 - b0, ld, psi, b->rho_w.ptr + b0, sbuf.ptr, ws.ptr, first, s);
             first = 0;
             b0 = b1;
         }
-        if (!first) b200::launch_rho_reduce_r<R>(g, nsplit, ws.ptr, rho, s);
+        if (!first) b200::launch_rho_reduce<R>(g, shape.nsplit, ws.ptr, rho, s);
         return;
     }
     const long N = g.nxyz();

@@ -255,8 +255,11 @@ class Server {
   private:
     size_t outstanding() const { return queue_.size() + size_t(inflight_); }
 
+    // a slot's stick buffer: many slots share the budget, so a slot takes less than a lone H|psi> caller would
+    static constexpr size_t kSlotStickBytes = size_t(48) << 20;
+
     // device bytes of one solver slot: Davidson buffers (FP64 engine, plus the FP32 engine when mixed),
-    // start vectors, and the H|psi> scratch (stick-buffer chunk of at most ~48 MB, becp / ps)
+    // start vectors, and the H|psi> scratch (a stick-buffer chunk, becp / ps)
     size_t slot_bytes(int cell, int nb, int precision) const {
         const ServeCell& c = cells_[cell];
         const size_t nbx = size_t(ndim_) * nb, d = size_t(c.dim_max), d32 = d + (d & 1);
@@ -271,7 +274,7 @@ class Server {
             b += engine(8, d32) + size_t(nb) * c.npwx * 8 + size_t(16) * 2 * nb * nbx * 4 + 2 * (nbx + 1) * nb * 8;
         const PWGrid& g = *c.h->h->grid;
         const size_t per_band = size_t(g.nst) * g.nz * 16;
-        b += std::max(per_band, std::min(per_band * nb, size_t(48) << 20)) + per_band;
+        b += std::max(per_band, std::min(per_band * nb, kSlotStickBytes)) + per_band;
         b += size_t(c.nkb + 1) * nb * 16 * 4 + (size_t(16) << 20);
         // FP64 projector products on the int8 tensor cores: psi residues (2 real rows per band, one byte per
         // modulus and real entry) and the per-modulus product residues of H psi
@@ -391,6 +394,7 @@ class Server {
         slot->dav->set_stream(slot->stream.s);
         slot->psi.resize(size_t(r.nbands) * c.npwx);
         slot->work = std::make_unique<HpsiWork>();
+        slot->work->stick_bytes = kSlotStickBytes;
         slot->bytes = slot_bytes(r.cell, r.nbands, r.precision);
         return slot;
     }

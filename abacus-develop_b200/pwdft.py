@@ -473,12 +473,12 @@ class HamiltPW:
         return (best.value, var.value) if with_variant else best.value
 
     def set_chunk(self, chunk):
-        """Bands per stick-buffer chunk of the local pass (0: the 48 MB default rule)."""
+        """Bands per stick-buffer chunk of the local pass (0: the default rule, 512 MB of stick buffer)."""
         call("b200_hamilt_set_band_chunk", self._h, int(chunk))
 
     def set_plane_variant(self, variant):
-        """Plane pass of the register transforms (1: warp-shuffle lanes; 2-5: two-pass transforms; 0: default)
-        for every handle of this basis in this handle's precision."""
+        """Launch shape of the plane pass (0, 1: the best by the library's estimate, 2-5: the next ones) for every
+        handle of this basis in this handle's precision."""
         call("b200_hamilt_set_plane_variant", self._h, int(variant))
 
     def set_fp64_gemm(self, mode, nmods=16):

@@ -220,16 +220,16 @@ int b200_graph_capture_hpsi_kbatch(b200_hamilt* h, int nk, const int* iks, int s
 int b200_graph_launch(b200_graph* g, void* stream);
 int b200_graph_destroy(b200_graph* g);
 /* Times the kinetic + local pass of k-point ik over candidate band-chunk sizes (1, 2, 4 ... 128 and
- * nbands) and, on grids with square planes of 64, 96 or 128 points, over the plane-pass variants
+ * nbands) and, on grids with line transforms, over the plane-pass variants
  * (three timed repetitions each after one warm-up), and keeps the fastest pair: the chunk for this
  * handle, the plane variant for every handle of this basis in the handle's precision.  Overwrites
  * hpsi_d.  best_chunk / best_variant may be NULL.  No counterpart in the reference. */
 int b200_hamilt_autotune(b200_hamilt* h, int ik, int nbands, int ld, const void* psi_d, void* hpsi_d, void* stream,
                          int* best_chunk, int* best_variant);
-/* Plane pass of the local H|psi> on grids with square planes of 64, 96 or 128 points, for every
- * handle of this basis in this handle's precision: 1 = one warp per line, five warp-shuffle lane
- * stages; 2-5 = two-pass register transforms through shared memory (four launch shapes); 0 = the
- * default.  All variants give the same results within rounding.  No counterpart in the reference. */
+/* Launch shape (warps a CTA, rows a warp at a time) of the plane pass of the local H|psi> on grids with
+ * line transforms, for every handle of this basis in this handle's precision: 0 or 1 = the best by the
+ * library's estimate, 2-5 = the second to fifth best.  All variants give the same results.
+ * No counterpart in the reference. */
 int b200_hamilt_set_plane_variant(b200_hamilt* h, int variant);
 /* The FP64 projector products of Nonlocal::act (nonlocal_pw.cpp:255-276, becp = vkb^H psi and
  * H psi += vkb (D becp), here with D folded into the projectors) for this handle: on the int8 tensor
@@ -241,7 +241,7 @@ int b200_hamilt_set_plane_variant(b200_hamilt* h, int variant);
  * Rebuilds the projector forms of every k-point (synchronous). */
 int b200_hamilt_set_fp64_gemm(b200_hamilt* h, int mode, int nmods);
 /* Bands per stick-buffer chunk of this handle's local pass (0 = the default: the largest chunk whose
- * stick buffer stays within 48 MB).  What b200_hamilt_autotune sets.  No counterpart in the reference. */
+ * stick buffer stays within 512 MB; 48 MB in the slots of a server).  What b200_hamilt_autotune sets.  No counterpart in the reference. */
 int b200_hamilt_set_band_chunk(b200_hamilt* h, int chunk);
 
 /* ---- psi -> rho (ElecStatePW::psiToRho, module_elecstate/elecstate_pw.cpp:78-216) ---- */

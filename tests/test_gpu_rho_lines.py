@@ -1,0 +1,42 @@
+"""psi -> rho on the line transforms against the oracle's loop over bands (1e-12 relative in FP64, 2e-5 in FP32):
+square and rectangular planes, sums in shared memory and in the partial planes, bands without weight (skipped, also
+when they hold NaN), rho added to, more partial planes than a later run of bands fills."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from oracle import hamilt_ref as H
+from oracle.pw_basis_ref import PWBasisKRef
+
+CASES = [((18, 18, 18), 1), ((20, 25, 32), 7), ((36, 36, 45), 33), ((72, 36, 50), 4), ((96, 96, 27), 3), ((125, 125, 16), 2),
+         ((128, 128, 18), 3), ((144, 144, 16), 1), ((135, 64, 20), 2)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("grid,nb", CASES)
+def test_rho_matches_oracle(pkg, grid, nb, prec):
+    torch = pytest.importorskip("torch")
+    lat, k = np.diag(np.array(grid, dtype=float)), np.array([[0.125, -0.375, 0.375]])
+    b = pkg.pwdft.PWBasisK(0.28, lat, 30.0, k, grid=grid)
+    ref = PWBasisKRef(0.28, lat, 30.0, k, grid=grid)
+    rng = np.random.default_rng(5)
+    npw, ld = int(b.npwk[0]), int(b.npwk[0]) + 1
+    psi = np.zeros((nb, ld), dtype=np.complex128)
+    psi[:, :npw] = rng.standard_normal((nb, npw)) + 1j * rng.standard_normal((nb, npw))
+    w = rng.uniform(0.1, 2.0, size=nb)
+    rho0 = rng.uniform(0.0, 1.0, size=b.nxyz)
+    want = rho0.copy()
+    if nb > 4:
+        w[2] = w[nb - 2] = 0.0
+    for ib in range(nb):
+        if w[ib]:
+            want += w[ib] * np.abs(H.recip_to_real(ref, psi[ib, :npw], 0)) ** 2
+    if nb > 4:
+        psi[2] = np.nan
+    pd = torch.from_numpy(psi).to("cuda", torch.complex64 if prec else torch.complex128)
+    rho = torch.from_numpy(rho0).to("cuda", torch.float32 if prec else torch.float64)
+    b.psi_to_rho(0, pd, nb, ld, w, rho)
+    torch.cuda.synchronize()
+    assert np.max(np.abs(rho.cpu().numpy() - want)) / np.max(want) < (2e-5 if prec else 1e-12)
