@@ -263,38 +263,52 @@ __global__ void __launch_bounds__(256) k_oz_res_cols(int K, const double2* __res
 }
 
 // largest magnitude over row r of a column-major M x K matrix (one thread per row; coalesced along rows)
+// segment blockIdx.y of gridDim.y of the row -> part[row][segment]
 __global__ void k_oz_absmax_rows(int M, int K, const double2* __restrict__ X, long ld, double* __restrict__ part) {
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= M) return;
+    const int nseg = gridDim.y, sg = blockIdx.y;
+    const int k0 = int(long(K) * sg / nseg), k1 = int(long(K) * (sg + 1) / nseg);
     double m = 0.0;
-    for (int k = 0; k < K; ++k) m = oz_amax(m, X[r + long(k) * ld]);
-    part[r] = m;
+#pragma unroll 8
+    for (int k = k0; k < k1; ++k) m = oz_amax(m, X[r + long(k) * ld]);
+    part[long(r) * nseg + sg] = m;
 }
 
 // residues of the rows of a column-major M x K matrix: a 32-row x 32-column tile per block (32 x 8 threads),
 // loaded along rows and written along K through shared memory
 __global__ void __launch_bounds__(256) k_oz_res_rows(int M, int K, const double2* __restrict__ X, long ld,
-                                                     const double* __restrict__ part, const __grid_constant__ OzConst c,
+                                                     const double* __restrict__ part, int nseg, const __grid_constant__ OzConst c,
                                                      signed char* __restrict__ res, long kp, long plane,
                                                      int* __restrict__ exps) {
     __shared__ __align__(16) unsigned char tile[kOzMaxMods][32][72];
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int r0 = blockIdx.y * 32, k0 = blockIdx.x * 32;
     const int row = r0 + tx;
-    const int e = row < M ? oz_exponent(part[row], c.q) : 0;
+    double mx = 0.0;
+    if (row < M)
+        for (int t = 0; t < nseg; ++t) mx = fmax(mx, part[long(row) * nseg + t]);
+    const int e = row < M ? oz_exponent(mx, c.q) : 0;
     if (blockIdx.x == 0 && ty == 0 && row < M) exps[row] = e;
     const bool bad = e == kOzNonFinite;
     const OzScale scale(bad ? 0 : e);
-    for (int kk = ty; kk < 32; kk += 8) {
-        const int k = k0 + kk;
-        const double2 x = (row < M && k < K && !bad) ? X[row + long(k) * ld] : make_double2(0.0, 0.0);
-        const unsigned long long ur = scale(x.x), ui = scale(x.y);
+    // four consecutive k a thread, so that a modulus's residues go to shared memory as one 8-byte word
+    unsigned long long ur[4], ui[4];
 #pragma unroll
-        for (int l = 0; l < kOzMaxMods; ++l) {
-            if (l >= c.n) break;
-            tile[l][tx][2 * kk] = (unsigned char)oz_sym(oz_res(ur, c, l), c.h[l]);
-            tile[l][tx][2 * kk + 1] = (unsigned char)oz_sym(oz_res(ui, c, l), c.h[l]);
-        }
+    for (int t = 0; t < 4; ++t) {
+        const int k = k0 + 4 * ty + t;
+        const double2 x = (row < M && k < K && !bad) ? X[row + long(k) * ld] : make_double2(0.0, 0.0);
+        ur[t] = scale(x.x);
+        ui[t] = scale(x.y);
+    }
+#pragma unroll
+    for (int l = 0; l < kOzMaxMods; ++l) {
+        if (l >= c.n) break;
+        unsigned w[2] = {0, 0};
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+            w[t / 2] |= (oz_sym(oz_res(ur[t], c, l), c.h[l]) | (oz_sym(oz_res(ui[t], c, l), c.h[l]) << 8)) << (16 * (t % 2));
+        *reinterpret_cast<uint2*>(&tile[l][tx][8 * ty]) = make_uint2(w[0], w[1]);
     }
     __syncthreads();
     const int t = ty * 32 + tx;
@@ -823,11 +837,12 @@ void oz_prepare_a(char opa, int M, int K, const double2* A, int lda, int nmods, 
     out.n = nmods;
     out.res.resize(size_t(nmods) * M * out.kp);
     out.exps.resize(size_t(M));
-    w.part.resize(size_t(M));
-    k_oz_absmax_rows<<<(M + 127) / 128, 128, 0, s>>>(M, K, A, lda, w.part.ptr);
+    const int nseg = K >= 64 ? 4 : 1;  // four CTAs a row block: 423 MB in 70 us instead of 170 with one
+    w.part.resize(size_t(M) * nseg);
+    k_oz_absmax_rows<<<dim3((M + 127) / 128, nseg), 128, 0, s>>>(M, K, A, lda, w.part.ptr);
     launch_check();
     B200_CHECK((M + 31) / 32 <= 65535, kInvalidArgument, "int8 GEMM: too many rows");
-    k_oz_res_rows<<<dim3((K + 31) / 32, (M + 31) / 32), dim3(32, 8), 0, s>>>(M, K, A, lda, w.part.ptr, c, out.res.ptr,
+    k_oz_res_rows<<<dim3((K + 31) / 32, (M + 31) / 32), dim3(32, 8), 0, s>>>(M, K, A, lda, w.part.ptr, nseg, c, out.res.ptr,
                                                                             out.kp, long(M) * out.kp, out.exps.ptr);
     launch_check();
 }
