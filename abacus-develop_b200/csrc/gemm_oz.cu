@@ -54,7 +54,8 @@ constexpr int kOzSmem = 227 * 1024;            // dynamic shared memory per CTA:
 struct OzConst {
     int n, q;  // q: set per call from K' (oz_scale_bits)
     unsigned m[kOzMaxMods], magic[kOzMaxMods];             // magic = ceil(2^32 / m)
-    unsigned c21[kOzMaxMods], c42[kOzMaxMods], off62[kOzMaxMods], c31[kOzMaxMods];
+    unsigned w0[kOzMaxMods], w1[kOzMaxMods];  // 256^i mod m, i = 0 .. 3 and 4 .. 7, a byte each
+    unsigned off62[kOzMaxMods], c31[kOzMaxMods];
     unsigned h[kOzMaxMods];  // residues are kept shifted by h: 128 for m = 256, (m - 1) / 2 for odd m
     double wa[kOzMaxMods], wb[kOzMaxMods];
     double mprod, log2m;
@@ -80,8 +81,10 @@ OzConst make_const(int n) {
         const unsigned m = unsigned(kOzMods[l]);
         c.m[l] = m;
         c.magic[l] = unsigned(((1ull << 32) + m - 1) / m);
-        c.c21[l] = unsigned((1ull << 21) % m);
-        c.c42[l] = unsigned((1ull << 42) % m);
+        for (int i = 0; i < 4; ++i) {
+            c.w0[l] |= unsigned((1ull << (8 * i)) % m) << (8 * i);
+            c.w1[l] |= unsigned((1ull << (8 * i + 32)) % m) << (8 * i);
+        }
         c.h[l] = m == 256 ? 128u : (m - 1) / 2;
         c.off62[l] = unsigned((m - (1ull << 62) % m + c.h[l]) % m);
         c.c31[l] = unsigned((1ull << 31) % m);
@@ -130,11 +133,19 @@ __device__ __forceinline__ unsigned oz_umod(unsigned x, unsigned m, unsigned mag
     const int r = int(x - q * m);
     return unsigned(r < 0 ? r + int(m) : r);
 }
-// (u - 2^62 + h) mod m for u < 2^63: three 21-bit pieces
-__device__ __forceinline__ unsigned oz_res(unsigned long long u, const OzConst& c, int l) {
-    if (l == 0) return (unsigned(u) + 128u) & 0xFFu;  // m_0 = 256 (h = 128): 2^62 = 0 mod 256
-    const unsigned p0 = unsigned(u) & 0x1FFFFFu, p1 = unsigned(u >> 21) & 0x1FFFFFu, p2 = unsigned(u >> 42);
-    return oz_umod(p2 * c.c42[l] + p1 * c.c21[l] + p0 + c.off62[l], c.m[l], c.magic[l]);
+// The symmetric representative of v = u - 2^62 modulo m (u < 2^63) in the low byte, the other bits undefined: in
+// [-128, 127] for m = 256, [-(m-1)/2, (m-1)/2] for odd m.  u = sum byte_i 256^i, so x = sum byte_i (256^i mod m) +
+// (h - 2^62) mod m < 2^20 by two four-byte dot products; ceil(2^32 / m) then gives floor(x / m) exactly (the excess
+// is below x / 2^32 < 1 / m), and r - h with r = x mod m is v's representative.  Two dot products, a high and a low
+// multiply and an add a residue, where three 21-bit pieces took four multiplies, a correction and a mask.
+__device__ __forceinline__ unsigned oz_byte(unsigned long long u, const OzConst& c, int l) {
+    if (l == 0) return unsigned(u);  // m_0 = 256, 2^62 = 0 mod 256
+    const unsigned x = __dp4a(unsigned(u), c.w0[l], __dp4a(unsigned(u >> 32), c.w1[l], c.off62[l]));
+    return x - c.h[l] - __umulhi(x, c.magic[l]) * c.m[l];
+}
+// the low bytes of a, b, c, d as one word
+__device__ __forceinline__ unsigned oz_pack(unsigned a, unsigned b, unsigned c, unsigned d) {
+    return __byte_perm(__byte_perm(a, b, 0x0040), __byte_perm(c, d, 0x0040), 0x5410);
 }
 // x 2^e rounded to the nearest integer, offset by 2^62 (|x| 2^e < 2^62): two exact scalings by powers of two
 // (2^e itself may lie outside the double range), then one rounding conversion
@@ -150,11 +161,6 @@ struct OzScale {
         return (unsigned long long)(__double2ll_rn((x * s1) * s2) + (1ll << 62));
     }
 };
-// the symmetric representative (as a byte) of v, and of -v, from r = (v + h) mod m: r - h lies in
-// [-128, 127] for m = 256 and in [-(m-1)/2, (m-1)/2] for odd m; h - r is -v's (128 = -128 as a byte, m = 256)
-__device__ __forceinline__ unsigned oz_sym(unsigned r, unsigned h) { return (r - h) & 0xFFu; }
-__device__ __forceinline__ unsigned oz_symneg(unsigned r, unsigned h) { return (h - r) & 0xFFu; }
-
 // exponent e of a row whose largest magnitude is mx: mx 2^e < 2^q (kOzNonFinite for NaN / infinity)
 __device__ __forceinline__ int oz_exponent(double mx, int q) {
     if (!(mx <= 1.7976931348623157e308)) return kOzNonFinite;
@@ -229,31 +235,25 @@ __global__ void __launch_bounds__(256) k_oz_res_cols(int K, const double2* __res
 #pragma unroll
         for (int l = 0; l < kOzMaxMods; ++l) {
             if (l >= c.n) break;
-            const unsigned hs = c.h[l];
             unsigned rr[4], ri[4];
 #pragma unroll
             for (int t = 0; t < 4; ++t) {
-                rr[t] = oz_res(ur[t], c, l);
-                ri[t] = oz_res(ui[t], c, l);
+                rr[t] = oz_byte(ur[t], c, l);
+                ri[t] = oz_byte(ui[t], c, l);
             }
             signed char* pl = res + long(l) * plane + 2 * kb;
             if (KIND == 0) {
-                uint2 v;
-                v.x = oz_sym(rr[0], hs) | (oz_sym(ri[0], hs) << 8) | (oz_sym(rr[1], hs) << 16) | (oz_sym(ri[1], hs) << 24);
-                v.y = oz_sym(rr[2], hs) | (oz_sym(ri[2], hs) << 8) | (oz_sym(rr[3], hs) << 16) | (oz_sym(ri[3], hs) << 24);
-                *reinterpret_cast<uint2*>(pl + long(j) * kp) = v;
+                *reinterpret_cast<uint2*>(pl + long(j) * kp) =
+                    make_uint2(oz_pack(rr[0], ri[0], rr[1], ri[1]), oz_pack(rr[2], ri[2], rr[3], ri[3]));
             } else {
+                // -v's representative is the negative (128 = -128 as a byte, m = 256)
                 uint2 vre, vim;
                 if (KIND == 1) {  // re = [br, -bi], im = [bi, br]
-                    vre.x = oz_sym(rr[0], hs) | (oz_symneg(ri[0], hs) << 8) | (oz_sym(rr[1], hs) << 16) | (oz_symneg(ri[1], hs) << 24);
-                    vre.y = oz_sym(rr[2], hs) | (oz_symneg(ri[2], hs) << 8) | (oz_sym(rr[3], hs) << 16) | (oz_symneg(ri[3], hs) << 24);
-                    vim.x = oz_sym(ri[0], hs) | (oz_sym(rr[0], hs) << 8) | (oz_sym(ri[1], hs) << 16) | (oz_sym(rr[1], hs) << 24);
-                    vim.y = oz_sym(ri[2], hs) | (oz_sym(rr[2], hs) << 8) | (oz_sym(ri[3], hs) << 16) | (oz_sym(rr[3], hs) << 24);
+                    vre = make_uint2(oz_pack(rr[0], 0u - ri[0], rr[1], 0u - ri[1]), oz_pack(rr[2], 0u - ri[2], rr[3], 0u - ri[3]));
+                    vim = make_uint2(oz_pack(ri[0], rr[0], ri[1], rr[1]), oz_pack(ri[2], rr[2], ri[3], rr[3]));
                 } else {  // re = [br, bi], im = [bi, -br]
-                    vre.x = oz_sym(rr[0], hs) | (oz_sym(ri[0], hs) << 8) | (oz_sym(rr[1], hs) << 16) | (oz_sym(ri[1], hs) << 24);
-                    vre.y = oz_sym(rr[2], hs) | (oz_sym(ri[2], hs) << 8) | (oz_sym(rr[3], hs) << 16) | (oz_sym(ri[3], hs) << 24);
-                    vim.x = oz_sym(ri[0], hs) | (oz_symneg(rr[0], hs) << 8) | (oz_sym(ri[1], hs) << 16) | (oz_symneg(rr[1], hs) << 24);
-                    vim.y = oz_sym(ri[2], hs) | (oz_symneg(rr[2], hs) << 8) | (oz_sym(ri[3], hs) << 16) | (oz_symneg(rr[3], hs) << 24);
+                    vre = make_uint2(oz_pack(rr[0], ri[0], rr[1], ri[1]), oz_pack(rr[2], ri[2], rr[3], ri[3]));
+                    vim = make_uint2(oz_pack(ri[0], 0u - rr[0], ri[1], 0u - rr[1]), oz_pack(ri[2], 0u - rr[2], ri[3], 0u - rr[3]));
                 }
                 *reinterpret_cast<uint2*>(pl + long(2 * j) * kp) = vre;
                 *reinterpret_cast<uint2*>(pl + long(2 * j + 1) * kp) = vim;
@@ -304,11 +304,13 @@ __global__ void __launch_bounds__(256) k_oz_res_rows(int M, int K, const double2
 #pragma unroll
     for (int l = 0; l < kOzMaxMods; ++l) {
         if (l >= c.n) break;
-        unsigned w[2] = {0, 0};
+        unsigned rr[4], ri[4];
 #pragma unroll
-        for (int t = 0; t < 4; ++t)
-            w[t / 2] |= (oz_sym(oz_res(ur[t], c, l), c.h[l]) | (oz_sym(oz_res(ui[t], c, l), c.h[l]) << 8)) << (16 * (t % 2));
-        *reinterpret_cast<uint2*>(&tile[l][tx][8 * ty]) = make_uint2(w[0], w[1]);
+        for (int t = 0; t < 4; ++t) {
+            rr[t] = oz_byte(ur[t], c, l);
+            ri[t] = oz_byte(ui[t], c, l);
+        }
+        *reinterpret_cast<uint2*>(&tile[l][tx][8 * ty]) = make_uint2(oz_pack(rr[0], ri[0], rr[1], ri[1]), oz_pack(rr[2], ri[2], rr[3], ri[3]));
     }
     __syncthreads();
     const int t = ty * 32 + tx;
