@@ -352,6 +352,15 @@ template <> struct Blas<double2> {
 };
 }  // namespace
 
+bool Hamilt::small_products(int ik, int nb, int nk) const {
+    const NonlocalK& k = nl[ik];
+    return fp64_gemm == 1 && !(k.oz_ready && nb >= kOzMinBands) && proj_small(k.nkb, nb, grid->kmaps[ik].npw, nk);
+}
+
+// whether the projection of a block runs on the side stream: below about a million points of local work the two
+// events and two waits cost more than the overlap gives
+static bool project_beside(long nxyz, long columns) { return nxyz * columns > 1000000; }
+
 template <typename T>
 void Hamilt::hpsi(int ik, int spin, int nb, int ld, const T* psi, T* hpsi, int mode, cudaStream_t s, HpsiWork* wk) {
     using R = typename RealOf<T>::type;
@@ -413,6 +422,9 @@ void Hamilt::hpsi(int ik, int spin, int nb, int ld, const T* psi, T* hpsi, int m
     B200_CHECK(k.folded, kInvalidArgument, "projectors and D not both set for this k-point");
     const T* vkbd = f64 ? reinterpret_cast<const T*>(k.vkbd.ptr + size_t(spin) * nkb * k.npwx)
                         : reinterpret_cast<const T*>(k.vkbdf.ptr + size_t(spin) * nkb * k.ldf);
+    const bool small = f64 && !oz && small_products(ik, nb, 1);
+    ProjEntry pe{};
+    if constexpr (f64) pe = ProjEntry{k.vkb.ptr, vkbd, psi, hpsi, npw, k.npwx};
     const bool oz = f64 && k.oz_ready && (fp64_gemm == 2 || (fp64_gemm == 1 && nb >= kOzMinBands));
     if (oz) W.tcw.ensure();  // the int8 GEMM reports a bounded wait that ran out in the same error word
     auto projections = [&](cudaStream_t st) {
@@ -420,6 +432,10 @@ void Hamilt::hpsi(int ik, int spin, int nb, int ld, const T* psi, T* hpsi, int m
             if (oz) {
                 oz_zgemm('C', nkb, nb, npw, one, k.vkb_oz, psi, ld, zero, becp, nkb, W.ozw, W.tcw.err.ptr, st);
                 return;
+            if (small) {
+                proj_becp(&pe, 1, nkb, nb, ld, becp, W.pjw, st);
+                return;
+            }
             }
             B200_CUBLAS(cublasSetStream(cublas, st));
             B200_CUBLAS(Blas<T>::gemm(cublas, CUBLAS_OP_C, CUBLAS_OP_N, nkb, nb, npw, &one, (const T*)k.vkb.ptr, k.npwx,
@@ -430,6 +446,9 @@ void Hamilt::hpsi(int ik, int spin, int nb, int ld, const T* psi, T* hpsi, int m
             int ldb = ld;
             if (ld & 1) {  // the TMA row pitch must be a multiple of 16 bytes: stage psi with an even pitch
                 ldb = ld + 1;
+    } else if (!project_beside(grid->nxyz(), nb)) {
+        projections(s);
+        local_pass(s);
                 psi_pad32.resize(size_t(nb) * ldb);
                 B200_CUDA(cudaMemcpy2DAsync(psi_pad32.ptr, size_t(ldb) * sizeof(float2), psi, size_t(ld) * sizeof(float2),
                                             size_t(npw) * sizeof(float2), nb, cudaMemcpyDeviceToDevice, st));
@@ -444,6 +463,8 @@ void Hamilt::hpsi(int ik, int spin, int nb, int ld, const T* psi, T* hpsi, int m
         // the projection runs on a second stream beside the local pass (it reads psi only); H psi += vkbd becp
         // waits for both
         W.ensure_side();
+        } else if (small) {
+            proj_add(&pe, 1, nkb, nb, ld, becp, s);
         B200_CUDA(cudaEventRecord(W.ev_fork, s));
         B200_CUDA(cudaStreamWaitEvent(W.side, W.ev_fork, 0));
         projections(W.side);
@@ -510,6 +531,14 @@ void Hamilt::hpsi_nc(int ik, int nb, int ld, const T* psi, T* hpsi, cudaStream_t
     const int nkb = k.nkb;
     const T one = cmake<T>(1, 0), zero = cmake<T>(0, 0);
     T* becp;
+        } else if (fp64_gemm == 1 && proj_small(nkb, 2 * nb, npw, 1)) {
+            ProjEntry pe{k.vkb.ptr, nullptr, psi, hpsi, npw, k.npwx};
+            proj_becp(&pe, 1, nkb, 2 * nb, ld, becp, W.pjw, s);
+            for (int half = 0; half < 2; ++half) {
+                pe.vkbd = k.wnc.ptr + size_t(half) * 2 * nkb * k.npwx;
+                pe.hpsi = hpsi + size_t(half) * ld;
+                proj_add(&pe, 1, 2 * nkb, nb, 2 * ld, becp, s);
+            }
     if constexpr (f64) {
         W.becp64.resize(size_t(2) * nkb * nb);
         becp = W.becp64.ptr;
@@ -590,8 +619,42 @@ void Hamilt::hpsi_kbatch(int nk, const int* iks, int spin, int nb, int ld, const
         W.sb32.resize(size_t(nk) * chunk * grid->nst * grid->nz);
         sb = W.sb32.ptr;
     }
-    if (!launch_hpsi_local_kbatch_lines<T, R>(*grid, args, nk, nb, veff, sb, chunk, grid->basis.tpiba2, s)) {
-        for (int q = 0; q < nk; ++q) hpsi<T>(iks[q], spin, nb, ld, psis[q], hpsis[q], 1, s, &W);
+    auto local_pass = [&] {
+        if (!launch_hpsi_local_kbatch_lines<T, R>(*grid, args, nk, nb, veff, sb, chunk, grid->basis.tpiba2, s))
+            for (int q = 0; q < nk; ++q) hpsi<T>(iks[q], spin, nb, ld, psis[q], hpsis[q], 1, s, &W);
+    };
+    if constexpr (f64) {
+        // small products: all k-points in one launch each, becp beside the local pass
+        const int nkb = nl[iks[0]].nkb;
+        bool batch = nkb > 0 && nb > 0 && deeq.ptr && spin >= 0 && spin < nspin;
+        for (int q = 0; q < nk && batch; ++q) {
+            const NonlocalK& k = nl[iks[q]];
+            batch = k.nkb == nkb && k.folded && small_products(iks[q], nb, nk);
+        }
+        if (batch) {
+            std::vector<ProjEntry> pe(nk);
+            for (int q = 0; q < nk; ++q) {
+                const NonlocalK& k = nl[iks[q]];
+                pe[q] = ProjEntry{k.vkb.ptr, k.vkbd.ptr + size_t(spin) * nkb * k.npwx, psis[q], hpsis[q],
+    local_pass();
+                                  grid->kmaps[iks[q]].npw, k.npwx};
+            }
+            W.becp64.resize(size_t(nk) * nkb * nb);
+            if (project_beside(grid->nxyz(), long(nk) * nb)) {
+                W.ensure_side();
+                B200_CUDA(cudaEventRecord(W.ev_fork, s));
+                B200_CUDA(cudaStreamWaitEvent(W.side, W.ev_fork, 0));
+                proj_becp(pe.data(), nk, nkb, nb, ld, W.becp64.ptr, W.pjw, W.side);
+                B200_CUDA(cudaEventRecord(W.ev_join, W.side));
+                local_pass();
+                B200_CUDA(cudaStreamWaitEvent(s, W.ev_join, 0));
+            } else {
+                proj_becp(pe.data(), nk, nkb, nb, ld, W.becp64.ptr, W.pjw, s);
+                local_pass();
+            }
+            proj_add(pe.data(), nk, nkb, nb, ld, W.becp64.ptr, s);
+            return;
+        }
     }
     for (int q = 0; q < nk; ++q) hpsi<T>(iks[q], spin, nb, ld, psis[q], hpsis[q], 2, s, &W);
 }

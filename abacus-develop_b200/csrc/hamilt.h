@@ -6,6 +6,7 @@
 
 #include "common.h"
 #include "gemm_oz.h"
+#include "proj_f64.h"
 #include "gemm_tc.h"
 #include "linalg_status.h"
 #include "pw_grid.h"
@@ -47,6 +48,7 @@ struct HpsiWork {
     DeviceArray<float2> sb32, becp32, psi_pad32, rb32;  // rb: real-space planes of the npol = 2 local pass
     cublasHandle_t cublas = nullptr;
     TcGemmWorkspace tcw;
+    ProjWorkspace pjw;  // FP64 projector products of small blocks
     OzWorkspace ozw;  // the FP64 projector products on the int8 tensor cores (psi / becp residues, products)
     // second stream of an H|psi>: the projections (becp, D becp) run on it beside the local pass
     cudaStream_t side = nullptr;
@@ -99,7 +101,8 @@ struct Hamilt {
     int chunk_override = 0;  // bands per stick-buffer chunk chosen by the autotuner (0 = the scratch's stick_bytes)
     // FP64 projector products: 0 = cuBLAS ZGEMM; int8 tensor cores (exact modular emulation, oz_mods moduli)
     // 1 = for calls of at least kOzMinBands bands (each call reads the projectors' whole residue form, twice the
-    // bytes of the FP64 projectors, so narrow calls go to cuBLAS, whose cost scales with the bands), 2 = always
+    // bytes of the FP64 projectors, so narrow calls go to cuBLAS, or if small to proj_f64.cu, whose cost scales with
+    // the bands), 2 = always
     int fp64_gemm = 1;
     static constexpr int kOzMinBands = 48;
     int oz_mods = 16;
@@ -128,6 +131,8 @@ struct Hamilt {
     // band b's components at psi + (2 b + c) ld, c = 0, 1
     template <typename T>
     void hpsi_nc(int ik, int nb, int ld, const T* psi, T* hpsi, cudaStream_t s, HpsiWork* w = nullptr);
+    // whether the FP64 projector products of nb bands of k-point ik (of a batch of nk) run on proj_f64.cu's kernels
+    bool small_products(int ik, int nb, int nk) const;
     // choose the FP64 projector products (0 cuBLAS, 1 int8 tensor cores from kOzMinBands bands, 2 int8 always;
     // nmods moduli) and re-fold
     void set_fp64_gemm(int mode, int nmods);

@@ -1,0 +1,301 @@
+// FP64 projector products of small blocks (nonlocal_pw.cpp:211-304): becp = vkb^H psi and H psi += vkbd becp, all
+// k-points of a batch in one launch each.
+//
+// Both are built from mma.sync m8n8k4 in FP64 (B200 has no tcgen05 FP64 kind; these instructions reach its FP64
+// peak), a complex product as four real ones.  Fragments come straight from global memory: a lane's A or B value is one complex
+// number (16 bytes: the real and imaginary parts of the fragment at once), four lanes cover 64 contiguous bytes of a
+// row (becp: both operands; H psi: becp) or eight cover 128 (H psi: vkbd), and the next step's values are loaded
+// before the current one is used.
+//   becp:  a warp owns 8 JT x 8 NT values of becp and a share of the plane waves; the four warps of a CTA and then
+//          the `slices` CTAs of a tile are added in a fixed order (the tile's last CTA reads the others' partial sums).
+//   H psi: a warp owns 8 NT bands x 16 plane waves, all projectors.
+#include <algorithm>
+#include <cmath>
+
+#include "proj_f64.h"
+
+namespace b200 {
+
+namespace {
+
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+                 : "+d"(c[0]), "+d"(c[1])
+                 : "d"(a), "d"(b));
+}
+// c += a b (CONJ: conj(a) b) for 8 x 8 complex tiles
+template <bool CONJ> __device__ __forceinline__ void zmma(double (&re)[2], double (&im)[2], double2 a, double2 b) {
+    dmma(re, a.x, b.x);
+    dmma(re, CONJ ? a.y : -a.y, b.y);
+    dmma(im, a.x, b.y);
+    dmma(im, CONJ ? -a.y : a.y, b.x);
+}
+
+struct OneProj {
+    ProjEntry e;
+    __device__ __forceinline__ const ProjEntry& get(int) const { return e; }
+};
+struct ManyProj {
+    ProjEntry e[kMaxProjBatch];
+    __device__ __forceinline__ const ProjEntry& get(int q) const { return e[q]; }
+};
+
+constexpr int kWarps = 4;
+
+// grid: x = projector tile + slice * tiles, y = band tile, z = k-point
+template <int JT, int NT, typename Src>
+__global__ void __launch_bounds__(kWarps * 32) k_proj_becp(Src src, int nkb, int nb, int ld, int jtiles, int slices,
+                                                          double2* __restrict__ becp, double2* __restrict__ part,
+                                                          unsigned* __restrict__ count) {
+    __shared__ double2 red[kWarps - 1][JT * NT * 64];
+    __shared__ bool last;
+    const ProjEntry& e = src.get(blockIdx.z);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int jt = blockIdx.x % jtiles, sl = blockIdx.x / jtiles;
+    const int j0 = jt * 8 * JT, b0 = blockIdx.y * 8 * NT;
+    const int r = lane >> 2, q = lane & 3;
+    // this warp's plane waves, in steps of 4: warp w of slice sl takes a run of whole steps
+    const int steps = (e.npw + 3) / 4, share = slices * kWarps, wi = sl * kWarps + warp;
+    const int t0 = int(long(steps) * wi / share), t1 = int(long(steps) * (wi + 1) / share);
+    const double2 *pa[JT], *pb[NT];
+    bool va[JT], vb[NT];
+#pragma unroll
+    for (int i = 0; i < JT; ++i) {
+        va[i] = j0 + 8 * i + r < nkb;
+        pa[i] = e.vkb + size_t(va[i] ? j0 + 8 * i + r : 0) * e.npwx + q;
+    }
+#pragma unroll
+    for (int i = 0; i < NT; ++i) {
+        vb[i] = b0 + 8 * i + r < nb;
+        pb[i] = e.psi + size_t(vb[i] ? b0 + 8 * i + r : 0) * ld + q;
+    }
+    double re[JT][NT][2], im[JT][NT][2];
+#pragma unroll
+    for (int i = 0; i < JT; ++i)
+#pragma unroll
+        for (int j = 0; j < NT; ++j) re[i][j][0] = re[i][j][1] = im[i][j][0] = im[i][j][1] = 0.0;
+    const double2 zero = make_double2(0.0, 0.0);
+    double2 a[2][JT], b[2][NT];
+    auto load = [&](int t, double2 (&x)[JT], double2 (&y)[NT]) {
+        const bool in = t < t1 && 4 * t + q < e.npw;
+#pragma unroll
+        for (int i = 0; i < JT; ++i) x[i] = in && va[i] ? __ldg(pa[i] + 4 * t) : zero;
+#pragma unroll
+        for (int i = 0; i < NT; ++i) y[i] = in && vb[i] ? __ldg(pb[i] + 4 * t) : zero;
+    };
+    auto use = [&](double2 (&x)[JT], double2 (&y)[NT]) {
+#pragma unroll
+        for (int i = 0; i < JT; ++i)
+#pragma unroll
+            for (int j = 0; j < NT; ++j) zmma<true>(re[i][j], im[i][j], x[i], y[j]);
+    };
+    load(t0, a[0], b[0]);
+    for (int t = t0; t < t1; t += 2) {
+        load(t + 1, a[1], b[1]);
+        use(a[0], b[0]);
+        load(t + 2, a[0], b[0]);
+        use(a[1], b[1]);
+    }
+    // the warps of the CTA, then the slices of the tile
+    auto at = [&](int i, int j, int h) { return (i * NT + j) * 64 + r * 8 + 2 * q + h; };
+    if (warp > 0) {
+#pragma unroll
+        for (int i = 0; i < JT; ++i)
+#pragma unroll
+            for (int j = 0; j < NT; ++j)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) red[warp - 1][at(i, j, h)] = make_double2(re[i][j][h], im[i][j][h]);
+    }
+    __syncthreads();
+    constexpr int TILE = JT * NT * 64;
+    const size_t tile = (size_t(blockIdx.z) * gridDim.y + blockIdx.y) * jtiles + jt;
+    double2* mine = part + (tile * slices + sl) * TILE;
+    if (warp == 0) {
+#pragma unroll
+        for (int i = 0; i < JT; ++i)
+#pragma unroll
+            for (int j = 0; j < NT; ++j)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    double2 v = make_double2(re[i][j][h], im[i][j][h]);
+#pragma unroll
+                    for (int w = 0; w < kWarps - 1; ++w) {
+                        const double2 o = red[w][at(i, j, h)];
+                        v.x += o.x;
+                        v.y += o.y;
+                    }
+                    if (slices > 1) {
+                        mine[at(i, j, h)] = v;
+                    } else {
+                        const int jj = j0 + 8 * i + r, bb = b0 + 8 * j + 2 * q + h;
+                        if (jj < nkb && bb < nb) becp[(size_t(blockIdx.z) * nb + bb) * nkb + jj] = v;
+                    }
+                }
+    }
+    if (slices == 1) return;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        last = atomicAdd(count + tile, 1u) == unsigned(slices - 1);
+        if (last) count[tile] = 0;  // for the next launch
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (int i = threadIdx.x; i < TILE; i += kWarps * 32) {
+        const double2* p = part + tile * slices * TILE + i;
+        double2 v = __ldcg(p);
+#pragma unroll 8
+        for (int s = 1; s < slices; ++s) {
+            const double2 o = __ldcg(p + size_t(s) * TILE);
+            v.x += o.x;
+            v.y += o.y;
+        }
+        const int ij = i >> 6, jj = j0 + 8 * (ij / NT) + ((i >> 3) & 7), bb = b0 + 8 * (ij % NT) + (i & 7);
+        if (jj < nkb && bb < nb) becp[(size_t(blockIdx.z) * nb + bb) * nkb + jj] = v;
+    }
+}
+
+// grid: x = plane-wave tile of 16 kWarps, y = band tile, z = k-point
+template <int NT, typename Src>
+__global__ void __launch_bounds__(kWarps * 32) k_proj_add(Src src, int nkb, int nb, int ld,
+                                                         const double2* __restrict__ becp) {
+    const ProjEntry& e = src.get(blockIdx.z);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int g0 = (blockIdx.x * kWarps + warp) * 16, b0 = blockIdx.y * 8 * NT;
+    if (g0 >= e.npw) return;
+    const int r = lane >> 2, q = lane & 3;
+    const double2* pa[NT];
+    bool va[NT], vb[2];
+#pragma unroll
+    for (int i = 0; i < NT; ++i) {
+        va[i] = b0 + 8 * i + r < nb;
+        pa[i] = becp + (size_t(blockIdx.z) * nb + (va[i] ? b0 + 8 * i + r : 0)) * nkb + q;
+    }
+    const double2* pb = e.vkbd + size_t(q) * e.npwx + g0 + r;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) vb[i] = g0 + 8 * i + r < e.npw;
+    const double2 zero = make_double2(0.0, 0.0);
+    // H psi of this tile first: its loads run beside the products
+    double2 h[NT][2][2];
+#pragma unroll
+    for (int i = 0; i < NT; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const int bb = b0 + 8 * i + r, g = g0 + 8 * j + 2 * q + k;
+                h[i][j][k] = bb < nb && g < e.npw ? e.hpsi[size_t(bb) * ld + g] : zero;
+            }
+    double re[NT][2][2], im[NT][2][2];
+#pragma unroll
+    for (int i = 0; i < NT; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) re[i][j][0] = re[i][j][1] = im[i][j][0] = im[i][j][1] = 0.0;
+    double2 a[2][NT], b[2][2];
+    const int steps = (nkb + 3) / 4;
+    auto load = [&](int t, double2 (&x)[NT], double2 (&y)[2]) {
+        const bool in = 4 * t + q < nkb;
+#pragma unroll
+        for (int i = 0; i < NT; ++i) x[i] = in && va[i] ? __ldg(pa[i] + 4 * t) : zero;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) y[i] = in && vb[i] ? __ldg(pb + size_t(4 * t) * e.npwx + 8 * i) : zero;
+    };
+    auto use = [&](double2 (&x)[NT], double2 (&y)[2]) {
+#pragma unroll
+        for (int i = 0; i < NT; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) zmma<false>(re[i][j], im[i][j], x[i], y[j]);
+    };
+    load(0, a[0], b[0]);
+    for (int t = 0; t < steps; t += 2) {
+        load(t + 1, a[1], b[1]);
+        use(a[0], b[0]);
+        load(t + 2, a[0], b[0]);
+        use(a[1], b[1]);
+    }
+#pragma unroll
+    for (int i = 0; i < NT; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const int bb = b0 + 8 * i + r, g = g0 + 8 * j + 2 * q + k;
+                if (bb < nb && g < e.npw)
+                    e.hpsi[size_t(bb) * ld + g] = make_double2(h[i][j][k].x + re[i][j][k], h[i][j][k].y + im[i][j][k]);
+            }
+}
+
+template <int JT, int NT, typename Src>
+void becp_launch(const Src& src, int nk, int nkb, int nb, int ld, int npw_max, double2* becp, ProjWorkspace& w,
+                 cudaStream_t s) {
+    const int jtiles = ceil_div(nkb, 8 * JT), btiles = ceil_div(nb, 8 * NT);
+    const long tiles = long(nk) * jtiles * btiles;
+    // slices of the plane waves: at most three CTAs a SM; a step of a warp (4 plane waves) costs about twice what the
+    // last CTA takes to add a slice, so a single tile's time is least near sqrt(steps / 2) slices
+    const int slices = int(std::max(1.0, std::min(double(ceil_div(444, tiles)), std::sqrt(npw_max / 8.0))));
+    if (slices > 1) {
+        w.part.resize(size_t(tiles) * slices * JT * NT * 64);
+        if (w.count.n < size_t(tiles)) {
+            w.count.resize(size_t(tiles));
+            B200_CUDA(cudaMemsetAsync(w.count.ptr, 0, w.count.n * sizeof(unsigned), s));
+        }
+    }
+    k_proj_becp<JT, NT, Src><<<dim3(jtiles * slices, btiles, nk), kWarps * 32, 0, s>>>(src, nkb, nb, ld, jtiles, slices, becp,
+                                                                                      w.part.ptr, w.count.ptr);
+    note_launch();
+    B200_CUDA(cudaGetLastError());
+}
+template <int NT, typename Src>
+void add_launch(const Src& src, int nk, int nkb, int nb, int ld, int npw_max, const double2* becp, cudaStream_t s) {
+    k_proj_add<NT, Src><<<dim3(ceil_div(npw_max, 16 * kWarps), ceil_div(nb, 8 * NT), nk), kWarps * 32, 0, s>>>(src, nkb, nb,
+                                                                                                             ld, becp);
+    note_launch();
+    B200_CUDA(cudaGetLastError());
+}
+
+// f(source of the k-points): by value, one or up to kMaxProjBatch
+template <typename F> void with_source(const ProjEntry* e, int nk, F&& f) {
+    B200_CHECK(nk >= 1 && nk <= kMaxProjBatch, kInvalidArgument, "projector products: 1..128 k-points a call");
+    if (nk == 1) {
+        OneProj o;
+        o.e = e[0];
+        f(o);
+    } else {
+        ManyProj m;
+        std::copy(e, e + nk, m.e);
+        f(m);
+    }
+}
+int npw_most(const ProjEntry* e, int nk) {
+    int m = 0;
+    for (int q = 0; q < nk; ++q) m = std::max(m, e[q].npw);
+    return m;
+}
+
+}  // namespace
+
+void proj_becp(const ProjEntry* e, int nk, int nkb, int nb, int ld, double2* becp, ProjWorkspace& w, cudaStream_t s) {
+    const int npw = npw_most(e, nk);
+    with_source(e, nk, [&](const auto& src) {
+        if (nb <= 8) becp_launch<4, 1>(src, nk, nkb, nb, ld, npw, becp, w, s);
+        else if (nb <= 16) becp_launch<4, 2>(src, nk, nkb, nb, ld, npw, becp, w, s);
+        else becp_launch<2, 4>(src, nk, nkb, nb, ld, npw, becp, w, s);
+    });
+}
+void proj_add(const ProjEntry* e, int nk, int nkb, int nb, int ld, const double2* becp, cudaStream_t s) {
+    const int npw = npw_most(e, nk);
+    with_source(e, nk, [&](const auto& src) {
+        if (nb <= 8) add_launch<1>(src, nk, nkb, nb, ld, npw, becp, s);
+        else if (nb <= 16) add_launch<2>(src, nk, nkb, nb, ld, npw, becp, s);
+        else add_launch<4>(src, nk, nkb, nb, ld, npw, becp, s);
+    });
+}
+
+// One k-point: both products, B200, the library's GEMMs against these (15 us of a call are its overhead): 16 projectors
+// x 380 plane waves, 8 bands 28 / 18 us, 47 bands 35 / 19; 64 x 3000, 4 bands 30 / 21, 12 bands 26 / 27; 128 x 9240, 8
+// bands 28 / 28, 24 bands 35 / 53.  A batch saves the library's calls for every k-point: 64 x (64 x 3000), 32 bands,
+// 1.18 ms against 0.36.
+bool proj_small(int nkb, int nb, int npw, int nk) { return double(nkb) * nb * npw <= (nk > 1 ? 2e7 : 3e6); }
+
+}  // namespace b200

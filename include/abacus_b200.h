@@ -236,7 +236,8 @@ int b200_hamilt_set_plane_variant(b200_hamilt* h, int variant);
  * cores (exact modular emulation of the FP64 product with nmods (12..16, default 16) moduli, as
  * b200_zgemm_i8) for H|psi> calls of at least 48 bands (mode 1, the default) or for every call (mode 2),
  * else cuBLAS ZGEMM (mode 0, and narrower calls in mode 1: the int8 path reads the projectors' whole
- * residue form per call).  Modes 1 and 2 keep the projectors also in residue form (2 x nmods bytes per
+ * residue form per call; in mode 1 small products, and batches of them, run on the library's own FP64
+ * tensor-core kernels).  Modes 1 and 2 keep the projectors also in residue form (2 x nmods bytes per
  * projector entry and spin) and each H|psi> caller about 6 x nmods bytes per psi entry of scratch.
  * Rebuilds the projector forms of every k-point (synchronous). */
 int b200_hamilt_set_fp64_gemm(b200_hamilt* h, int mode, int nmods);
