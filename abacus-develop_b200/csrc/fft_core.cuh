@@ -28,8 +28,16 @@ template <typename T> __host__ __device__ __forceinline__ T cmake(typename RealO
     r.y = y;
     return r;
 }
-template <typename T> __device__ __forceinline__ T cadd(T a, T b) { return cmake<T>(a.x + b.x, a.y + b.y); }
-template <typename T> __device__ __forceinline__ T csub(T a, T b) { return cmake<T>(a.x - b.x, a.y - b.y); }
+// FP32: sm_100 adds, multiplies and fuses two packed floats in one instruction (add / mul / fma .f32x2), so a complex
+// sum is one instruction; a difference is a fused b * (-1, -1) + a with the same rounding.
+template <typename T> __device__ __forceinline__ T cadd(T a, T b) {
+    if constexpr (sizeof(T) == 8) return __fadd2_rn(a, b);
+    else return cmake<T>(a.x + b.x, a.y + b.y);
+}
+template <typename T> __device__ __forceinline__ T csub(T a, T b) {
+    if constexpr (sizeof(T) == 8) return __ffma2_rn(b, make_float2(-1.f, -1.f), a);
+    else return cmake<T>(a.x - b.x, a.y - b.y);
+}
 template <typename T> __device__ __forceinline__ T cmul(T a, T b) {
     return cmake<T>(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
@@ -37,7 +45,22 @@ template <typename T> __device__ __forceinline__ T cmul(T a, T b) {
 template <typename T> __device__ __forceinline__ T cmulc(T a, T b) {
     return cmake<T>(a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y);
 }
-template <typename T> __device__ __forceinline__ T cscale(T a, typename RealOf<T>::type s) { return cmake<T>(a.x * s, a.y * s); }
+template <typename T> __device__ __forceinline__ T cscale(T a, typename RealOf<T>::type s) {
+    if constexpr (sizeof(T) == 8) return __fmul2_rn(a, make_float2(s, s));
+    else return cmake<T>(a.x * s, a.y * s);
+}
+// a * s + b, s real
+template <typename T> __device__ __forceinline__ T cfma(T a, typename RealOf<T>::type s, T b) {
+    if constexpr (sizeof(T) == 8) return __ffma2_rn(a, make_float2(s, s), b);
+    else return cmake<T>(fma(a.x, s, b.x), fma(a.y, s, b.y));
+}
+// the difference a - b with its parts exchanged, and m + i s a for a so exchanged: the quarter turn costs no moves,
+// its sign is in the factors
+template <typename T> __device__ __forceinline__ T csub_swap(T a, T b) { return cmake<T>(a.y - b.y, a.x - b.x); }
+template <typename T> __device__ __forceinline__ T cfma_i(T a, typename RealOf<T>::type s, T m) {
+    if constexpr (sizeof(T) == 8) return __ffma2_rn(a, make_float2(-s, s), m);
+    else return cmake<T>(fma(a.x, -s, m.x), fma(a.y, s, m.y));
+}
 // multiply by s*i, s = +1 or -1
 template <typename T, int S> __device__ __forceinline__ T cmul_si(T a) {
     return S > 0 ? cmake<T>(-a.y, a.x) : cmake<T>(a.y, -a.x);
@@ -62,43 +85,57 @@ template <typename T, int DIR> __device__ __forceinline__ void dft2(T* u) {
 
 template <typename T, int DIR> __device__ __forceinline__ void dft3(T* u) {
     using R = typename RealOf<T>::type;
-    const R s60 = R(0.86602540378443864676372317075294);  // sin(2 pi / 3)
+    const R s60 = R(DIR * 0.86602540378443864676372317075294);  // sin(2 pi / 3)
     const T t1 = cadd(u[1], u[2]);
-    const T t2 = cscale(cmul_si<T, DIR>(csub(u[1], u[2])), s60);
-    const T m = csub(u[0], cscale(t1, R(0.5)));
+    const T t2 = csub_swap(u[1], u[2]);
+    const T m = cfma(t1, R(-0.5), u[0]);
     u[0] = cadd(u[0], t1);
-    u[1] = cadd(m, t2);
-    u[2] = csub(m, t2);
+    u[1] = cfma_i(t2, s60, m);
+    u[2] = cfma_i(t2, -s60, m);
 }
 
 template <typename T, int DIR> __device__ __forceinline__ void dft4(T* u) {
+    using R = typename RealOf<T>::type;
     const T a0 = cadd(u[0], u[2]);
     const T a1 = csub(u[0], u[2]);
     const T b0 = cadd(u[1], u[3]);
-    const T b1 = cmul_si<T, DIR>(csub(u[1], u[3]));
-    u[0] = cadd(a0, b0);
     u[2] = csub(a0, b0);
-    u[1] = cadd(a1, b1);
-    u[3] = csub(a1, b1);
+    if constexpr (sizeof(T) == 8) {
+        const T b1 = csub_swap(u[1], u[3]);
+        u[1] = cfma_i(b1, R(DIR), a1);
+        u[3] = cfma_i(b1, R(-DIR), a1);
+    } else {
+        const T b1 = cmul_si<T, DIR>(csub(u[1], u[3]));
+        u[1] = cadd(a1, b1);
+        u[3] = csub(a1, b1);
+    }
+    u[0] = cadd(a0, b0);
 }
 
 template <typename T, int DIR> __device__ __forceinline__ void dft5(T* u) {
     using R = typename RealOf<T>::type;
-    const R c1 = R(0.30901699437494742410229341718282);   // cos(2 pi / 5)
-    const R c2 = R(-0.80901699437494742410229341718282);  // cos(4 pi / 5)
-    const R s1 = R(0.95105651629515357211643933337938);   // sin(2 pi / 5)
-    const R s2 = R(0.58778525229247312916870595463907);   // sin(4 pi / 5)
-    const T a1 = cadd(u[1], u[4]), b1 = csub(u[1], u[4]);
-    const T a2 = cadd(u[2], u[3]), b2 = csub(u[2], u[3]);
-    const T m1 = cadd(u[0], cadd(cscale(a1, c1), cscale(a2, c2)));
-    const T m2 = cadd(u[0], cadd(cscale(a1, c2), cscale(a2, c1)));
-    const T n1 = cmul_si<T, DIR>(cadd(cscale(b1, s1), cscale(b2, s2)));
-    const T n2 = cmul_si<T, DIR>(csub(cscale(b1, s2), cscale(b2, s1)));
+    const R c1 = R(0.30901699437494742410229341718282);         // cos(2 pi / 5)
+    const R c2 = R(-0.80901699437494742410229341718282);        // cos(4 pi / 5)
+    const R s1 = R(DIR * 0.95105651629515357211643933337938);   // sin(2 pi / 5)
+    const R s2 = R(DIR * 0.58778525229247312916870595463907);   // sin(4 pi / 5)
+    const T a1 = cadd(u[1], u[4]), b1 = csub_swap(u[1], u[4]);
+    const T a2 = cadd(u[2], u[3]), b2 = csub_swap(u[2], u[3]);
+    const T m1 = cfma(a2, c2, cfma(a1, c1, u[0]));
+    const T m2 = cfma(a2, c1, cfma(a1, c2, u[0]));
     u[0] = cadd(u[0], cadd(a1, a2));
-    u[1] = cadd(m1, n1);
-    u[4] = csub(m1, n1);
-    u[2] = cadd(m2, n2);
-    u[3] = csub(m2, n2);
+    if constexpr (sizeof(T) == 8) {
+        const T n1 = cfma(b2, s2, cscale(b1, s1));
+        const T n2 = cfma(b2, -s1, cscale(b1, s2));
+        u[1] = cfma_i(n1, R(1), m1);
+        u[4] = cfma_i(n1, R(-1), m1);
+        u[2] = cfma_i(n2, R(1), m2);
+        u[3] = cfma_i(n2, R(-1), m2);
+    } else {  // the same sums with the exchanged parts added directly
+        u[1] = cfma_i(b2, s2, cfma_i(b1, s1, m1));
+        u[4] = cfma_i(b2, -s2, cfma_i(b1, -s1, m1));
+        u[2] = cfma_i(b2, -s1, cfma_i(b1, s2, m2));
+        u[3] = cfma_i(b2, s1, cfma_i(b1, -s2, m2));
+    }
 }
 
 template <typename T, int DIR, int R> __device__ __forceinline__ void dftR(T* u) {

@@ -29,6 +29,7 @@
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
+#include <algorithm>
 #include <atomic>
 #include <mutex>
 
@@ -399,17 +400,31 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
 }
 
-// B (K x N complex, pitch ldb) -> hi = tf32 rounding, lo = B - hi, both with pitch ldh (even)
-__global__ void k_split_b(int K, int N, const float2* __restrict__ B, long ldb, float2* __restrict__ hi,
-                          float2* __restrict__ lo, long ldh) {
-    const long total = long(K) * N;
-    for (long t = blockIdx.x * long(blockDim.x) + threadIdx.x; t < total; t += long(gridDim.x) * blockDim.x) {
-        const long n = t / K, k = t - n * K;
+// B (K x N complex, any pitch ldb) -> hi = tf32 rounding, lo = B - hi, both with pitch ldh (even); column blockIdx.y
+// onwards, 256 entries a CTA and step (no division: 480 columns of 124 289, 477 MB in, 954 MB out)
+__global__ void __launch_bounds__(256) k_split_b(int K, int N, const float2* __restrict__ B, long ldb,
+                                                 float2* __restrict__ hi, float2* __restrict__ lo, long ldh) {
+    const int k = blockIdx.x * 256 + threadIdx.x;
+    if (k >= K) return;
+    for (long n = blockIdx.y; n < N; n += gridDim.y) {
         const float2 x = B[n * ldb + k];
         const float2 h = make_float2(tf32_round(x.x), tf32_round(x.y));
         hi[n * ldh + k] = h;
         lo[n * ldh + k] = make_float2(x.x - h.x, x.y - h.y);
     }
+}
+// B -> the same values with an even pitch
+__global__ void __launch_bounds__(256) k_pad_b(int K, int N, const float2* __restrict__ B, long ldb,
+                                               float2* __restrict__ out, long ldo) {
+    const int k = blockIdx.x * 256 + threadIdx.x;
+    if (k >= K) return;
+#pragma unroll 4
+    for (long n = blockIdx.y; n < N; n += gridDim.y) out[n * ldo + k] = B[n * ldb + k];
+}
+// about eight CTAs a SM, at least one column each
+dim3 column_grid(int K, int N) {
+    const int gx = ceil_div(K, 256);
+    return dim3(gx, std::max(1, std::min(std::min(N, 65535), ceil_div(148 * 16, gx))));
 }
 
 // C (+)= sum over splits, with alpha / beta, deterministic order
@@ -462,6 +477,9 @@ template <int BN, int OPA, int PRE> void set_attr_once() {
     });
 }
 
+// B is split once per call where many M tiles read it
+bool splits_b(int M) { return (2 * M + kBM - 1) / kBM >= 16; }
+
 template <int BN, int OPA>
 void launch(int M, int N, int K, float2 alpha, const float2* A, int lda, const float2* B, int ldb, float2 beta, float2* C,
             int ldc, TcGemmWorkspace& w, cudaStream_t s) {
@@ -471,17 +489,14 @@ void launch(int M, int N, int K, float2 alpha, const float2* A, int lda, const f
     const int tm = (M2 + kBM - 1) / kBM, tn = (N + BN - 1) / BN;
     // when many M tiles read B (tall op(A): the H|psi> and subspace updates), B is split into hi / lo once
     // here and the CTAs only copy it; otherwise every CTA splits its B tiles in shared memory
-    const bool pre = tm >= 16;
+    const bool pre = splits_b(M);
     CUtensorMap mB, mBl;
     if (pre) {
         const long ldh = long(K) + (K & 1);  // even: 16-byte row pitch
         w.bsplit.resize(size_t(2) * size_t(ldh) * N);
         float2* hi = w.bsplit.ptr;
         float2* lo = hi + size_t(ldh) * N;
-        const long total = long(K) * N;
-        int blocks = int((total + 255) / 256);
-        if (blocks > 148 * 8) blocks = 148 * 8;
-        k_split_b<<<blocks, 256, 0, s>>>(K, N, B, ldb, hi, lo, ldh);
+        k_split_b<<<column_grid(K, N), 256, 0, s>>>(K, N, B, ldb, hi, lo, ldh);
         note_launch();
         B200_CUDA(cudaGetLastError());
         mB = make_map(hi, 2L * K, N, 2L * ldh, 32, BN);
@@ -571,15 +586,11 @@ int TcGemmWorkspace::read_error(cudaStream_t s) {
 void set_tc_wait_limit_ns(unsigned long long ns) { g_wait_ns.store(ns ? ns : kWaitNs, std::memory_order_relaxed); }
 unsigned long long tc_wait_limit_ns() { return wait_limit_ns(); }
 
-void tc_cgemm(char opa, int M, int N, int K, float2 alpha, const float2* A, int lda, const float2* B, int ldb,
-              float2 beta, float2* C, int ldc, TcGemmWorkspace& w, cudaStream_t s) {
+static void run(char opa, int M, int N, int K, float2 alpha, const float2* A, int lda, const float2* B, int ldb, float2 beta,
+                float2* C, int ldc, TcGemmWorkspace& w, cudaStream_t s) {
     B200_CHECK(opa == 'N' || opa == 'C', kInvalidArgument, "tc_cgemm: op(A) must be 'N' or 'C'");
     B200_CHECK(M > 0 && N > 0 && K > 0, kInvalidArgument, "tc_cgemm: empty problem");
-    B200_CHECK(lda % 2 == 0 && ldb % 2 == 0, kInvalidArgument,
-               "tc_cgemm: lda and ldb must be even (16-byte row pitch for TMA)");
     B200_CHECK(ldc >= M, kInvalidArgument, "tc_cgemm: ldc < M");
-    B200_CHECK((reinterpret_cast<uintptr_t>(A) & 15) == 0 && (reinterpret_cast<uintptr_t>(B) & 15) == 0, kInvalidArgument,
-               "tc_cgemm: A and B must be 16-byte aligned");
     B200_CHECK(opa == 'C' ? lda >= K : lda >= M, kInvalidArgument, "tc_cgemm: lda too small");
     B200_CHECK(ldb >= K, kInvalidArgument, "tc_cgemm: ldb < K");
     w.ensure();
@@ -590,6 +601,36 @@ void tc_cgemm(char opa, int M, int N, int K, float2 alpha, const float2* A, int 
         if (opa == 'N') launch<128, 0>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, w, s);
         else launch<128, 1>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, w, s);
     }
+}
+
+void tc_cgemm(char opa, int M, int N, int K, float2 alpha, const float2* A, int lda, const float2* B, int ldb,
+              float2 beta, float2* C, int ldc, TcGemmWorkspace& w, cudaStream_t s) {
+    B200_CHECK(lda % 2 == 0 && ldb % 2 == 0, kInvalidArgument,
+               "tc_cgemm: lda and ldb must be even (16-byte row pitch for TMA)");
+    B200_CHECK((reinterpret_cast<uintptr_t>(A) & 15) == 0 && (reinterpret_cast<uintptr_t>(B) & 15) == 0, kInvalidArgument,
+               "tc_cgemm: A and B must be 16-byte aligned");
+    run(opa, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, w, s);
+}
+
+void tc_cgemm_any_ldb(char opa, int M, int N, int K, float2 alpha, const float2* A, int lda, const float2* B, int ldb,
+                      float2 beta, float2* C, int ldc, TcGemmWorkspace& w, cudaStream_t s) {
+    if (ldb % 2 == 0 || M <= 0 || N <= 0 || K <= 0) {
+        tc_cgemm(opa, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, w, s);
+        return;
+    }
+    B200_CHECK(ldb >= K, kInvalidArgument, "tc_cgemm: ldb < K");
+    if (splits_b(M)) {
+        B200_CHECK(lda % 2 == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0, kInvalidArgument,
+                   "tc_cgemm: A must be 16-byte aligned with an even pitch");
+        run(opa, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, w, s);
+        return;
+    }
+    const int ldp = K + (K & 1);
+    w.bpad.resize(size_t(N) * ldp);
+    k_pad_b<<<column_grid(K, N), 256, 0, s>>>(K, N, B, ldb, w.bpad.ptr, ldp);
+    note_launch();
+    B200_CUDA(cudaGetLastError());
+    tc_cgemm(opa, M, N, K, alpha, A, lda, w.bpad.ptr, ldp, beta, C, ldc, w, s);
 }
 
 }  // namespace b200

@@ -369,7 +369,6 @@ void Hamilt::hpsi(int ik, int spin, int nb, int ld, const T* psi, T* hpsi, int m
     auto& sb32 = W.sb32;
     auto& becp64 = W.becp64;
     auto& becp32 = W.becp32;
-    auto& psi_pad32 = W.psi_pad32;
     auto& tcw = W.tcw;
     cublasHandle_t cublas = W.cublas;
     constexpr bool f64 = std::is_same<T, double2>::value;
@@ -422,49 +421,38 @@ void Hamilt::hpsi(int ik, int spin, int nb, int ld, const T* psi, T* hpsi, int m
     B200_CHECK(k.folded, kInvalidArgument, "projectors and D not both set for this k-point");
     const T* vkbd = f64 ? reinterpret_cast<const T*>(k.vkbd.ptr + size_t(spin) * nkb * k.npwx)
                         : reinterpret_cast<const T*>(k.vkbdf.ptr + size_t(spin) * nkb * k.ldf);
+    const bool oz = f64 && k.oz_ready && (fp64_gemm == 2 || (fp64_gemm == 1 && nb >= kOzMinBands));
     const bool small = f64 && !oz && small_products(ik, nb, 1);
     ProjEntry pe{};
     if constexpr (f64) pe = ProjEntry{k.vkb.ptr, vkbd, psi, hpsi, npw, k.npwx};
-    const bool oz = f64 && k.oz_ready && (fp64_gemm == 2 || (fp64_gemm == 1 && nb >= kOzMinBands));
     if (oz) W.tcw.ensure();  // the int8 GEMM reports a bounded wait that ran out in the same error word
     auto projections = [&](cudaStream_t st) {
         if constexpr (f64) {
             if (oz) {
                 oz_zgemm('C', nkb, nb, npw, one, k.vkb_oz, psi, ld, zero, becp, nkb, W.ozw, W.tcw.err.ptr, st);
                 return;
+            }
             if (small) {
                 proj_becp(&pe, 1, nkb, nb, ld, becp, W.pjw, st);
                 return;
-            }
             }
             B200_CUBLAS(cublasSetStream(cublas, st));
             B200_CUBLAS(Blas<T>::gemm(cublas, CUBLAS_OP_C, CUBLAS_OP_N, nkb, nb, npw, &one, (const T*)k.vkb.ptr, k.npwx,
                                       psi, ld, &zero, becp, nkb));
         } else {
             // mixed precision: both projector products on the tensor cores (3xTF32)
-            const float2* psi_b = psi;
-            int ldb = ld;
-            if (ld & 1) {  // the TMA row pitch must be a multiple of 16 bytes: stage psi with an even pitch
-                ldb = ld + 1;
-    } else if (!project_beside(grid->nxyz(), nb)) {
-        projections(s);
-        local_pass(s);
-                psi_pad32.resize(size_t(nb) * ldb);
-                B200_CUDA(cudaMemcpy2DAsync(psi_pad32.ptr, size_t(ldb) * sizeof(float2), psi, size_t(ld) * sizeof(float2),
-                                            size_t(npw) * sizeof(float2), nb, cudaMemcpyDeviceToDevice, st));
-                psi_b = psi_pad32.ptr;
-            }
-            tc_cgemm('C', nkb, nb, npw, one, k.vkbf.ptr, k.ldf, psi_b, ldb, zero, becp, ldb_p, tcw, st);
+            tc_cgemm_any_ldb('C', nkb, nb, npw, one, k.vkbf.ptr, k.ldf, psi, ld, zero, becp, ldb_p, tcw, st);
         }
     };
     if (mode == 2) {
         projections(s);
+    } else if (!project_beside(grid->nxyz(), nb)) {
+        projections(s);
+        local_pass(s);
     } else {
         // the projection runs on a second stream beside the local pass (it reads psi only); H psi += vkbd becp
         // waits for both
         W.ensure_side();
-        } else if (small) {
-            proj_add(&pe, 1, nkb, nb, ld, becp, s);
         B200_CUDA(cudaEventRecord(W.ev_fork, s));
         B200_CUDA(cudaStreamWaitEvent(W.side, W.ev_fork, 0));
         projections(W.side);
@@ -475,6 +463,8 @@ void Hamilt::hpsi(int ik, int spin, int nb, int ld, const T* psi, T* hpsi, int m
     if constexpr (f64) {
         if (oz) {
             oz_zgemm('N', npw, nb, nkb, one, k.vkbd_oz[spin], becp, nkb, one, hpsi, ld, W.ozw, W.tcw.err.ptr, s);
+        } else if (small) {
+            proj_add(&pe, 1, nkb, nb, ld, becp, s);
         } else {
             B200_CUBLAS(cublasSetStream(cublas, s));
             B200_CUBLAS(Blas<T>::gemm(cublas, CUBLAS_OP_N, CUBLAS_OP_N, npw, nb, nkb, &one, vkbd, k.npwx, becp, nkb,
@@ -531,14 +521,6 @@ void Hamilt::hpsi_nc(int ik, int nb, int ld, const T* psi, T* hpsi, cudaStream_t
     const int nkb = k.nkb;
     const T one = cmake<T>(1, 0), zero = cmake<T>(0, 0);
     T* becp;
-        } else if (fp64_gemm == 1 && proj_small(nkb, 2 * nb, npw, 1)) {
-            ProjEntry pe{k.vkb.ptr, nullptr, psi, hpsi, npw, k.npwx};
-            proj_becp(&pe, 1, nkb, 2 * nb, ld, becp, W.pjw, s);
-            for (int half = 0; half < 2; ++half) {
-                pe.vkbd = k.wnc.ptr + size_t(half) * 2 * nkb * k.npwx;
-                pe.hpsi = hpsi + size_t(half) * ld;
-                proj_add(&pe, 1, 2 * nkb, nb, 2 * ld, becp, s);
-            }
     if constexpr (f64) {
         W.becp64.resize(size_t(2) * nkb * nb);
         becp = W.becp64.ptr;
@@ -549,6 +531,14 @@ void Hamilt::hpsi_nc(int ik, int nb, int ld, const T* psi, T* hpsi, cudaStream_t
             for (int half = 0; half < 2; ++half)
                 oz_zgemm('N', npw, nb, 2 * nkb, one, k.wnc_oz[half], becp, 2 * nkb, one, hpsi + size_t(half) * ld, 2 * ld,
                          W.ozw, W.tcw.err.ptr, s);
+        } else if (fp64_gemm == 1 && proj_small(nkb, 2 * nb, npw, 1)) {
+            ProjEntry pe{k.vkb.ptr, nullptr, psi, hpsi, npw, k.npwx};
+            proj_becp(&pe, 1, nkb, 2 * nb, ld, becp, W.pjw, s);
+            for (int half = 0; half < 2; ++half) {
+                pe.vkbd = k.wnc.ptr + size_t(half) * 2 * nkb * k.npwx;
+                pe.hpsi = hpsi + size_t(half) * ld;
+                proj_add(&pe, 1, 2 * nkb, nb, 2 * ld, becp, s);
+            }
         } else {
             B200_CUBLAS(cublasSetStream(W.cublas, s));
             const cuDoubleComplex* o = reinterpret_cast<const cuDoubleComplex*>(&one);
@@ -566,16 +556,7 @@ void Hamilt::hpsi_nc(int ik, int nb, int ld, const T* psi, T* hpsi, cudaStream_t
     } else {
         W.becp32.resize(size_t(2) * nkb * nb);
         becp = W.becp32.ptr;
-        const float2* psi_b = psi;
-        int ldb = ld;
-        if (ld & 1) {  // the TMA row pitch must be a multiple of 16 bytes: stage psi with an even pitch
-            ldb = ld + 1;
-            W.psi_pad32.resize(size_t(2) * nb * ldb);
-            B200_CUDA(cudaMemcpy2DAsync(W.psi_pad32.ptr, size_t(ldb) * sizeof(float2), psi, size_t(ld) * sizeof(float2),
-                                        size_t(npw) * sizeof(float2), 2 * nb, cudaMemcpyDeviceToDevice, s));
-            psi_b = W.psi_pad32.ptr;
-        }
-        tc_cgemm('C', nkb, 2 * nb, npw, one, k.vkbf.ptr, k.ldf, psi_b, ldb, zero, becp, nkb, W.tcw, s);
+        tc_cgemm_any_ldb('C', nkb, 2 * nb, npw, one, k.vkbf.ptr, k.ldf, psi, ld, zero, becp, nkb, W.tcw, s);
         for (int half = 0; half < 2; ++half)
             tc_cgemm('N', npw, nb, 2 * nkb, one, k.wncf.ptr + size_t(half) * 2 * nkb * k.ldf, k.ldf, becp, 2 * nkb, one,
                      hpsi + size_t(half) * ld, 2 * ld, W.tcw, s);
@@ -636,7 +617,6 @@ void Hamilt::hpsi_kbatch(int nk, const int* iks, int spin, int nb, int ld, const
             for (int q = 0; q < nk; ++q) {
                 const NonlocalK& k = nl[iks[q]];
                 pe[q] = ProjEntry{k.vkb.ptr, k.vkbd.ptr + size_t(spin) * nkb * k.npwx, psis[q], hpsis[q],
-    local_pass();
                                   grid->kmaps[iks[q]].npw, k.npwx};
             }
             W.becp64.resize(size_t(nk) * nkb * nb);
@@ -656,6 +636,7 @@ void Hamilt::hpsi_kbatch(int nk, const int* iks, int spin, int nb, int ld, const
             return;
         }
     }
+    local_pass();
     for (int q = 0; q < nk; ++q) hpsi<T>(iks[q], spin, nb, ld, psis[q], hpsis[q], 2, s, &W);
 }
 

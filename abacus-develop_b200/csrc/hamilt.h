@@ -45,7 +45,7 @@ struct NonlocalK {
 struct HpsiWork {
     size_t stick_bytes = kStickBytes;  // limit of a band chunk's stick buffer
     DeviceArray<double2> sb64, becp64, rb64;
-    DeviceArray<float2> sb32, becp32, psi_pad32, rb32;  // rb: real-space planes of the npol = 2 local pass
+    DeviceArray<float2> sb32, becp32, rb32;  // rb: real-space planes of the npol = 2 local pass
     cublasHandle_t cublas = nullptr;
     TcGemmWorkspace tcw;
     ProjWorkspace pjw;  // FP64 projector products of small blocks

@@ -2,7 +2,7 @@
 //
 // dft<T, DIR, Q>: Q-point DFT of u[0..Q) in place, natural order in and out (DIR +1: exp(+i), -1: exp(-i)).
 // Q = 2, 3, 4, 5 direct; 6, 10, 12, 15 by the prime-factor (Good-Thomas) map, which needs no twiddles
-// (12 = 3 x 4: 112 real operations against 136 with W_12 twiddles); 8, 9, 16, 25 as A x B with the twiddles
+// (12 = 3 x 4: 96 real operations against 120 with W_12 twiddles); 8, 9, 16, 25 as A x B with the twiddles
 // W_Q^j as exact constants (cos / sin of multiples of 2 pi / Q), the trivial ones folded at compile time.
 #pragma once
 #include "fft_core.cuh"

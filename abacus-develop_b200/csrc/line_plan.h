@@ -13,8 +13,8 @@ namespace line {
 
 // real operations of the register DFTs (adds, multiplies and FMAs; line_dft.cuh); 0: not built
 constexpr int dft_ops(int q) {
-    return q == 2 ? 4 : q == 3 ? 16 : q == 4 ? 16 : q == 5 ? 44 : q == 6 ? 44 : q == 8 ? 56 : q == 9 ? 114 : q == 10 ? 108
-         : q == 12 ? 112 : q == 15 ? 212 : q == 16 ? 168 : q == 25 ? 520 : 0;
+    return q == 2 ? 4 : q == 3 ? 12 : q == 4 ? 16 : q == 5 ? 36 : q == 6 ? 36 : q == 8 ? 56 : q == 9 ? 88 : q == 10 ? 92
+         : q == 12 ? 96 : q == 15 ? 168 : q == 16 ? 168 : q == 25 ? 424 : 0;
 }
 // lane slots a line takes in a warp whose lines have r threads each (32 / r lines a warp, the rest idle)
 constexpr double lane_slots(int r) { return 32.0 / (32 / r); }
