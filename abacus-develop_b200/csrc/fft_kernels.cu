@@ -595,6 +595,7 @@ void launch_hpsi_local_nc(const PWGrid& g, int ik, const R* veff4_zyx, int ncols
 template <typename T>
 void launch_recip_to_real(const PWGrid& g, int ik, const T* in, T* out, T* aux, int add, double factor, cudaStream_t s) {
     using R = typename RealOf<T>::type;
+    if (launch_box_lines<T>(g, ik, true, in, out, aux, add, factor, s)) return;
     const size_t N = size_t(g.nxyz());
     B200_CUDA(cudaMemsetAsync(aux, 0, N * sizeof(T), s));
     const size_t zs = zpass_smem(g, sizeof(T));
@@ -619,6 +620,7 @@ void launch_recip_to_real(const PWGrid& g, int ik, const T* in, T* out, T* aux, 
 
 template <typename T>
 void launch_real_to_recip(const PWGrid& g, int ik, const T* in, T* out, T* aux, int add, double factor, cudaStream_t s) {
+    if (launch_box_lines<T>(g, ik, false, in, out, aux, add, factor, s)) return;
     using R = typename RealOf<T>::type;
     const size_t xsm = size_t(2) * kBoxTile * odd_ld(g.nx) * sizeof(T);
     set_smem(k_box_x<T, R, -1>, xsm);

@@ -132,6 +132,8 @@ void build_line_plan(PWGrid& g) {
         p.x[i] = line::x_geom(nx, elem);
         p.y[i] = line::y_geom(ny, elem, p.x[i].r2 ? p.x[i].r2 : 1);
         p.z[i] = line::z_geom(nz, elem);
+        p.xbox[i] = line::z_geom(nx, elem);
+        p.ybox[i] = line::z_geom(ny, elem);
         if (!p.x[i].r1 || !p.y[i].r1 || !p.z[i].r1) return;
     }
     // occupied x: [0, xm) and [xh, nx)

@@ -84,6 +84,7 @@ struct PlaneShape {
 struct LinePlan {
     bool ok = false;
     LineGeom x[2], y[2], z[2];
+    LineGeom xbox[2], ybox[2];  // x and y lines whose threads are neighbours in the line index (box_lines.cu)
     int xm = 0, xh = 0, xoff = 0;
     std::vector<PlaneShape> shapes[2][2];
 };
@@ -167,6 +168,10 @@ template <typename T>
 void launch_recip_to_real(const PWGrid& g, int ik, const T* in, T* out, T* aux, int add, double factor, cudaStream_t s);
 template <typename T>
 void launch_real_to_recip(const PWGrid& g, int ik, const T* in, T* out, T* aux, int add, double factor, cudaStream_t s);
+// both on the line transforms (box_lines.cu); false (nothing launched) where they do not hold
+template <typename T>
+bool launch_box_lines(const PWGrid& g, int ik, bool inverse, const T* in, T* out, T* aux, int add, double factor,
+                      cudaStream_t s);
 // V_eff (ABACUS r order) -> (z, y, x) transposed copy, in precision R.
 template <typename R>
 void launch_transpose_veff(const PWGrid& g, const double* veff, R* out, cudaStream_t s);
