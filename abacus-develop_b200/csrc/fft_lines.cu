@@ -10,6 +10,8 @@ namespace {
 constexpr size_t kSmemMax = 227 * 1024;
 
 constexpr int kSMs = 148;
+// the class of a run-time r1 (RMAX of the kernels)
+int rmax_of(int r) { return r <= 10 ? 10 : r <= 16 ? 16 : 25; }
 
 // instructions of the busiest of nw warps with L rows at a time, from the operation counts (x transforms one way
 // only and no V_eff for inverse_only)
@@ -77,8 +79,6 @@ const PlaneShape& pick_shape(const std::vector<PlaneShape>& c, long nctas, int v
 using line::ManyK;
 using line::OneK;
 
-int rmax_of(int r) { return r <= 10 ? 10 : r <= 16 ? 16 : 25; }
-
 template <typename T, typename R, int NPOL>
 void plane_pass(const PWGrid& g, int nplanes, const R* v, T* sb, cudaStream_t s) {
     constexpr int pi = sizeof(T) == 8;
@@ -103,9 +103,9 @@ void z_pass(bool inv, const PWGrid& g, const Src& src, int nk, int b0, int nbc, 
     if (line::z_fixed<T, R, Src>(g, a)) return;
     const LineGeom& gz = g.lines.z[sizeof(T) == 8];
     switch (rmax_of(gz.r1)) {
-        case 10: line::z_launch<T, R, 10>(g, gz, a); break;
-        case 16: line::z_launch<T, R, 16>(g, gz, a); break;
-        default: line::z_launch<T, R, 25>(g, gz, a); break;
+        case 10: line::z_launch<T, R, 10, 128>(g, gz, a); break;
+        case 16: line::z_launch<T, R, 16, 128>(g, gz, a); break;
+        default: line::z_launch<T, R, 25, 128>(g, gz, a); break;
     }
 }
 

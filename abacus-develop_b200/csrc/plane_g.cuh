@@ -347,12 +347,15 @@ __global__ void __launch_bounds__(MAXT, 1) k_rho_g(PlaneMapView pm, GX gx, GY gy
     }
 }
 
-// ---- z passes: TS sticks per CTA ----
+// ---- z passes: TS sticks per CTA, ZT threads ----
+// Lines of 9 or 10 threads take 160, so that the 16 FP64 sticks of a CTA go through pass A in one round (with 128
+// threads the second round held 2 of 16 lines: forward pass at nz = 108, 120 bands, 78 us).
+constexpr int z_threads(int r2) { return r2 >= 9 ? 160 : 128; }
 // A stick's occupied z are one run modulo nz and its values consecutive in psi (stick descriptor: first value,
 // first z, count), so pass A reads psi, and writes H psi, directly.  Pass B's threads are neighbours in the
 // stick index, so the plane-major stick buffer is written and read in whole rows of TS sticks.
-template <typename T, int RMAX, int TS, typename Src, typename GZ>
-__global__ void __launch_bounds__(128, RMAX > 16 ? 2 : 4)
+template <typename T, int RMAX, int TS, int ZT, typename Src, typename GZ>
+__global__ void __launch_bounds__(ZT, RMAX > 16 ? 2 : ZT > 128 ? 3 : 4)
     k_zinv_g(Src src, GZ gz, int b0, int nbc, const T* __restrict__ roots, T* __restrict__ sb) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T* A = reinterpret_cast<T*>(smem_raw);
@@ -364,7 +367,7 @@ __global__ void __launch_bounds__(128, RMAX > 16 ? 2 : 4)
     const int band = blockIdx.y;
     const T* p = reinterpret_cast<const T*>(e.psi) + size_t(b0 + band) * e.ld;
     {
-        const int na = 128 / gz.r2, la = tid / gz.r2, ta = tid - la * gz.r2;
+        const int na = ZT / gz.r2, la = tid / gz.r2, ta = tid - la * gz.r2;
         for (int sl = la; sl < ns; sl += na) {
             if (la >= na) break;
             const int2 d = __ldg(sm.sd + s0 + sl);
@@ -389,7 +392,7 @@ __global__ void __launch_bounds__(128, RMAX > 16 ? 2 : 4)
     const int sl = tid % TS;
     if (sl >= ns) return;
     T* out = sb + (size_t(blockIdx.z) * nbc + band) * gz.n * sm.nst + s0 + sl;
-    for (int k1 = tid / TS; k1 < gz.r1; k1 += 128 / TS) {
+    for (int k1 = tid / TS; k1 < gz.r1; k1 += ZT / TS) {
         const T* blk = A + sl * gz.ld + k1 * gz.rs;
         with_r2<RMAX>(gz, [&](auto q) {
             constexpr int Q = decltype(q)::value;
@@ -404,8 +407,8 @@ __global__ void __launch_bounds__(128, RMAX > 16 ? 2 : 4)
     }
 }
 
-template <typename T, typename R, int RMAX, int TS, typename Src, typename GZ>
-__global__ void __launch_bounds__(128, RMAX > 16 ? 2 : 4)
+template <typename T, typename R, int RMAX, int TS, int ZT, typename Src, typename GZ>
+__global__ void __launch_bounds__(ZT, RMAX > 16 ? 2 : ZT > 128 ? 3 : 4)
     k_zfwd_g(Src src, GZ gz, int b0, int nbc, const T* __restrict__ roots, const T* __restrict__ sb, R tpiba2,
              R invn, int accumulate) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -419,7 +422,7 @@ __global__ void __launch_bounds__(128, RMAX > 16 ? 2 : 4)
     const T* p = reinterpret_cast<const T*>(e.psi) + size_t(b0 + band) * e.ld;
     T* h = reinterpret_cast<T*>(e.hpsi) + size_t(b0 + band) * e.ld;
     const R* gk2 = reinterpret_cast<const R*>(e.gk2);
-    const int na = 128 / gz.r2, la = tid / gz.r2, ta = tid - la * gz.r2;
+    const int na = ZT / gz.r2, la = tid / gz.r2, ta = tid - la * gz.r2;
     // psi and |k+G|^2 of this thread's line of pass A; with compiled lines those of the first line are loaded
     // before the stick buffer is read, so that both latencies overlap
     constexpr int kR1 = MaxR1<GZ, RMAX>::value;
@@ -449,7 +452,7 @@ __global__ void __launch_bounds__(128, RMAX > 16 ? 2 : 4)
     {
         const int sl = tid % TS;
         const T* in = sb + (size_t(blockIdx.z) * nbc + band) * gz.n * sm.nst + s0 + sl;
-        for (int k1 = tid / TS; k1 < gz.r1; k1 += 128 / TS) {
+        for (int k1 = tid / TS; k1 < gz.r1; k1 += ZT / TS) {
             if (sl >= ns) break;
             T* blk = A + sl * gz.ld + k1 * gz.rs;
             with_r2<RMAX>(gz, [&](auto q) {
@@ -493,7 +496,7 @@ __global__ void __launch_bounds__(128, RMAX > 16 ? 2 : 4)
             });
         }
     if (!accumulate && blockIdx.x == 0)
-        for (int g = e.npw + tid; g < e.ld; g += 128) h[g] = zero_of<T>();
+        for (int g = e.npw + tid; g < e.ld; g += ZT) h[g] = zero_of<T>();
 }
 
 }  // namespace line

@@ -8,7 +8,9 @@ namespace b200 {
 namespace line {
 
 // threads of a CTA, and resident threads of an SM, by the registers the transforms need: FP64 lines of 12 points and
-// more in pass A take 168 a thread (96^2: 12 warps of 168 run the local pass in 1.53 ms, 16 of 128 in 1.56)
+// more in pass A take 168 a thread, the others 128.  Plane pass with fewer and more: 96^2 FP64 (12 x 8) 12 warps of 168
+// 1.17 ms, 16 of 128 1.20; 72 x 36 FP64 16 of 128 284 us, 20 of 96 365, 12 of 168 339; 36^2 FP64 16 of 128 658 us,
+// 24 of 80 730, 12 of 168 657; 96^2 FP32 16 of 128 580 us, 20 of 96 610, 12 of 168 614.
 constexpr int plane_threads(size_t elem, int r1) { return elem == 8 || r1 <= 10 ? 512 : r1 <= 16 ? 384 : 256; }
 
 template <typename T> const T* roots_of(const FftAxis& a) {
@@ -99,19 +101,19 @@ template <typename T, typename Src> struct ZArgs {
 };
 template <typename T> constexpr int z_tile() { return sizeof(T) == 16 ? 16 : 32; }  // 256 bytes of a plane row
 
-template <typename T, typename R, int RMAX, typename Src, typename GZ>
+template <typename T, typename R, int RMAX, int ZT, typename Src, typename GZ>
 void z_launch(const PWGrid& g, GZ gz, const ZArgs<T, Src>& a) {
     constexpr int TS = z_tile<T>();
     const size_t smem = size_t(TS) * gz.ld * sizeof(T);
     const dim3 grid(ceil_div(g.nst, TS), a.nbc, a.nk);
     if (a.inv) {
-        auto kern = k_zinv_g<T, RMAX, TS, Src, GZ>;
+        auto kern = k_zinv_g<T, RMAX, TS, ZT, Src, GZ>;
         set_smem(kern, smem);
-        kern<<<grid, 128, smem, a.s>>>(a.src, gz, a.b0, a.nbc, roots_of<T>(g.az), a.sb);
+        kern<<<grid, ZT, smem, a.s>>>(a.src, gz, a.b0, a.nbc, roots_of<T>(g.az), a.sb);
     } else {
-        auto kern = k_zfwd_g<T, R, RMAX, TS, Src, GZ>;
+        auto kern = k_zfwd_g<T, R, RMAX, TS, ZT, Src, GZ>;
         set_smem(kern, smem);
-        kern<<<grid, 128, smem, a.s>>>(a.src, gz, a.b0, a.nbc, roots_of<T>(g.az), a.sb, R(a.tpiba2),
+        kern<<<grid, ZT, smem, a.s>>>(a.src, gz, a.b0, a.nbc, roots_of<T>(g.az), a.sb, R(a.tpiba2),
                                        R(1.0 / double(g.nxyz())), a.accumulate);
     }
     note_launch();
@@ -119,7 +121,7 @@ void z_launch(const PWGrid& g, GZ gz, const ZArgs<T, Src>& a) {
 }
 template <typename T, typename R, int N, typename Src> bool z_fixed_n(const PWGrid& g, const ZArgs<T, Src>& a) {
     constexpr LineGeom z = z_geom(N, sizeof(T));
-    z_launch<T, R, z.r1>(g, FixedGeom<N, z.r1, z.r2, z.rs, z.ld>(), a);
+    z_launch<T, R, z.r1, z_threads(z.r2)>(g, FixedGeom<N, z.r1, z.r2, z.rs, z.ld>(), a);
     return true;
 }
 // the z passes with lines of nz compiled in; false for other grids (zpass_f64.cu, zpass_f32.cu, and *_many)
