@@ -142,6 +142,7 @@ _SIGS = {
 }
 
 _lib = None
+_torch = None
 
 
 class B200Error(RuntimeError):
@@ -216,6 +217,15 @@ def ptr(t) -> int:
 
 
 def stream_ptr(stream=None):
-    import torch
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return s.cuda_stream
+    """Raw pointer of a stream, by default the current stream of the current device (read without building a
+    torch Stream object: 0.8 us instead of 3.4 on every call of a functor)."""
+    if stream is not None:
+        return stream.cuda_stream
+    global _torch
+    if _torch is None:
+        import torch
+        _torch = torch
+    cuda = _torch.cuda
+    if not cuda.is_initialized():
+        return cuda.current_stream().cuda_stream
+    return _torch._C._cuda_getCurrentRawStream(cuda.current_device())
