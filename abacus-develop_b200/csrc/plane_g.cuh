@@ -349,13 +349,14 @@ __global__ void __launch_bounds__(MAXT, 1) k_rho_g(PlaneMapView pm, GX gx, GY gy
 
 // ---- z passes: TS sticks per CTA, ZT threads ----
 // Lines of 9 or 10 threads take 160, so that the 16 FP64 sticks of a CTA go through pass A in one round (with 128
-// threads the second round held 2 of 16 lines: forward pass at nz = 108, 120 bands, 78 us).
-constexpr int z_threads(int r2) { return r2 >= 9 ? 160 : 128; }
+// threads the second round held 2 of 16 lines: forward pass at nz = 108, 120 bands, 78 us, now 65); lines of 5 or 6 take
+// 96, all of them busy and more CTAs resident (nz = 36, 2048 bands: 151 us, now 124).
+constexpr int z_threads(int r2) { return r2 >= 9 ? 160 : r2 >= 7 || r2 <= 4 ? 128 : 96; }
 // A stick's occupied z are one run modulo nz and its values consecutive in psi (stick descriptor: first value,
 // first z, count), so pass A reads psi, and writes H psi, directly.  Pass B's threads are neighbours in the
 // stick index, so the plane-major stick buffer is written and read in whole rows of TS sticks.
 template <typename T, int RMAX, int TS, int ZT, typename Src, typename GZ>
-__global__ void __launch_bounds__(ZT, RMAX > 16 ? 2 : ZT > 128 ? 3 : 4)
+__global__ void __launch_bounds__(ZT, RMAX > 16 ? 2 : 512 / ZT)
     k_zinv_g(Src src, GZ gz, int b0, int nbc, const T* __restrict__ roots, T* __restrict__ sb) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T* A = reinterpret_cast<T*>(smem_raw);
@@ -408,7 +409,7 @@ __global__ void __launch_bounds__(ZT, RMAX > 16 ? 2 : ZT > 128 ? 3 : 4)
 }
 
 template <typename T, typename R, int RMAX, int TS, int ZT, typename Src, typename GZ>
-__global__ void __launch_bounds__(ZT, RMAX > 16 ? 2 : ZT > 128 ? 3 : 4)
+__global__ void __launch_bounds__(ZT, RMAX > 16 ? 2 : 512 / ZT)
     k_zfwd_g(Src src, GZ gz, int b0, int nbc, const T* __restrict__ roots, const T* __restrict__ sb, R tpiba2,
              R invn, int accumulate) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
