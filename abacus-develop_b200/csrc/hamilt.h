@@ -100,7 +100,7 @@ struct Hamilt {
     HpsiWork work;  // default scratch for callers that do not bring their own
     int chunk_override = 0;  // bands per stick-buffer chunk chosen by the autotuner (0 = the scratch's stick_bytes)
     // FP64 projector products: 0 = cuBLAS ZGEMM; int8 tensor cores (exact modular emulation, oz_mods moduli)
-    // 1 = for calls of at least kOzMinBands bands (each call reads the projectors' whole residue form, twice the
+    // 1 = for calls of at least kOzMinBands bands that proj_f64.cu does not run faster (each call reads the projectors' whole residue form, twice the
     // bytes of the FP64 projectors, so narrow calls go to cuBLAS, or if small to proj_f64.cu, whose cost scales with
     // the bands), 2 = always
     int fp64_gemm = 1;
@@ -133,6 +133,8 @@ struct Hamilt {
     void hpsi_nc(int ik, int nb, int ld, const T* psi, T* hpsi, cudaStream_t s, HpsiWork* w = nullptr);
     // whether the FP64 projector products of nb bands of k-point ik (of a batch of nk) run on proj_f64.cu's kernels
     bool small_products(int ik, int nb, int nk) const;
+    // whether the products of a call of nb bands (`columns` columns of psi) run on the int8 tensor cores
+    bool int8_products(bool ready, int nkb, int nb, int columns, int npw) const;
     // choose the FP64 projector products (0 cuBLAS, 1 int8 tensor cores from kOzMinBands bands, 2 int8 always;
     // nmods moduli) and re-fold
     void set_fp64_gemm(int mode, int nmods);

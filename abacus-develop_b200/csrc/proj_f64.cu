@@ -8,7 +8,7 @@
 // before the current one is used.
 //   becp:  a warp owns 8 JT x 8 NT values of becp and a share of the plane waves; the four warps of a CTA and then
 //          the `slices` CTAs of a tile are added in a fixed order (the tile's last CTA reads the others' partial sums).
-//   H psi: a warp owns 8 NT bands x 16 plane waves, all projectors.
+//   H psi: a warp owns 8 NT bands x 8 GT plane waves, all projectors.
 #include <algorithm>
 #include <cmath>
 
@@ -156,17 +156,17 @@ __global__ void __launch_bounds__(kWarps * 32) k_proj_becp(Src src, int nkb, int
     }
 }
 
-// grid: x = plane-wave tile of 16 kWarps, y = band tile, z = k-point
-template <int NT, typename Src>
+// grid: x = plane-wave tile of 8 GT kWarps, y = band tile, z = k-point
+template <int NT, int GT, typename Src>
 __global__ void __launch_bounds__(kWarps * 32) k_proj_add(Src src, int nkb, int nb, int ld,
                                                          const double2* __restrict__ becp) {
     const ProjEntry& e = src.get(blockIdx.z);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int g0 = (blockIdx.x * kWarps + warp) * 16, b0 = blockIdx.y * 8 * NT;
+    const int g0 = (blockIdx.x * kWarps + warp) * 8 * GT, b0 = blockIdx.y * 8 * NT;
     if (g0 >= e.npw) return;
     const int r = lane >> 2, q = lane & 3;
     const double2* pa[NT];
-    bool va[NT], vb[2];
+    bool va[NT], vb[GT];
 #pragma unroll
     for (int i = 0; i < NT; ++i) {
         va[i] = b0 + 8 * i + r < nb;
@@ -174,38 +174,38 @@ __global__ void __launch_bounds__(kWarps * 32) k_proj_add(Src src, int nkb, int 
     }
     const double2* pb = e.vkbd + size_t(q) * e.npwx + g0 + r;
 #pragma unroll
-    for (int i = 0; i < 2; ++i) vb[i] = g0 + 8 * i + r < e.npw;
+    for (int i = 0; i < GT; ++i) vb[i] = g0 + 8 * i + r < e.npw;
     const double2 zero = make_double2(0.0, 0.0);
     // H psi of this tile first: its loads run beside the products
-    double2 h[NT][2][2];
+    double2 h[NT][GT][2];
 #pragma unroll
     for (int i = 0; i < NT; ++i)
 #pragma unroll
-        for (int j = 0; j < 2; ++j)
+        for (int j = 0; j < GT; ++j)
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
                 const int bb = b0 + 8 * i + r, g = g0 + 8 * j + 2 * q + k;
                 h[i][j][k] = bb < nb && g < e.npw ? e.hpsi[size_t(bb) * ld + g] : zero;
             }
-    double re[NT][2][2], im[NT][2][2];
+    double re[NT][GT][2], im[NT][GT][2];
 #pragma unroll
     for (int i = 0; i < NT; ++i)
 #pragma unroll
-        for (int j = 0; j < 2; ++j) re[i][j][0] = re[i][j][1] = im[i][j][0] = im[i][j][1] = 0.0;
-    double2 a[2][NT], b[2][2];
+        for (int j = 0; j < GT; ++j) re[i][j][0] = re[i][j][1] = im[i][j][0] = im[i][j][1] = 0.0;
+    double2 a[2][NT], b[2][GT];
     const int steps = (nkb + 3) / 4;
-    auto load = [&](int t, double2 (&x)[NT], double2 (&y)[2]) {
+    auto load = [&](int t, double2 (&x)[NT], double2 (&y)[GT]) {
         const bool in = 4 * t + q < nkb;
 #pragma unroll
         for (int i = 0; i < NT; ++i) x[i] = in && va[i] ? __ldg(pa[i] + 4 * t) : zero;
 #pragma unroll
-        for (int i = 0; i < 2; ++i) y[i] = in && vb[i] ? __ldg(pb + size_t(4 * t) * e.npwx + 8 * i) : zero;
+        for (int i = 0; i < GT; ++i) y[i] = in && vb[i] ? __ldg(pb + size_t(4 * t) * e.npwx + 8 * i) : zero;
     };
-    auto use = [&](double2 (&x)[NT], double2 (&y)[2]) {
+    auto use = [&](double2 (&x)[NT], double2 (&y)[GT]) {
 #pragma unroll
         for (int i = 0; i < NT; ++i)
 #pragma unroll
-            for (int j = 0; j < 2; ++j) zmma<false>(re[i][j], im[i][j], x[i], y[j]);
+            for (int j = 0; j < GT; ++j) zmma<false>(re[i][j], im[i][j], x[i], y[j]);
     };
     load(0, a[0], b[0]);
     for (int t = 0; t < steps; t += 2) {
@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(kWarps * 32) k_proj_add(Src src, int nkb, int 
 #pragma unroll
     for (int i = 0; i < NT; ++i)
 #pragma unroll
-        for (int j = 0; j < 2; ++j)
+        for (int j = 0; j < GT; ++j)
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
                 const int bb = b0 + 8 * i + r, g = g0 + 8 * j + 2 * q + k;
@@ -231,9 +231,9 @@ void becp_launch(const Src& src, int nk, int nkb, int nb, int ld, int npw_max, d
                  cudaStream_t s) {
     const int jtiles = ceil_div(nkb, 8 * JT), btiles = ceil_div(nb, 8 * NT);
     const long tiles = long(nk) * jtiles * btiles;
-    // slices of the plane waves: at most three CTAs a SM; a step of a warp (4 plane waves) costs about twice what the
+    // slices of the plane waves: one wave of three CTAs a SM; a step of a warp (4 plane waves) costs about twice what the
     // last CTA takes to add a slice, so a single tile's time is least near sqrt(steps / 2) slices
-    const int slices = int(std::max(1.0, std::min(double(ceil_div(444, tiles)), std::sqrt(npw_max / 8.0))));
+    const int slices = int(std::max(1.0, std::min(double(std::max<long>(1, 444 / tiles)), std::sqrt(npw_max / 8.0))));
     if (slices > 1) {
         w.part.resize(size_t(tiles) * slices * JT * NT * 64);
         if (w.count.n < size_t(tiles)) {
@@ -246,12 +246,21 @@ void becp_launch(const Src& src, int nk, int nkb, int nb, int ld, int npw_max, d
     note_launch();
     B200_CUDA(cudaGetLastError());
 }
-template <int NT, typename Src>
-void add_launch(const Src& src, int nk, int nkb, int nb, int ld, int npw_max, const double2* becp, cudaStream_t s) {
-    k_proj_add<NT, Src><<<dim3(ceil_div(npw_max, 16 * kWarps), ceil_div(nb, 8 * NT), nk), kWarps * 32, 0, s>>>(src, nkb, nb,
-                                                                                                             ld, becp);
+template <int NT, int GT, typename Src>
+void add_run(const Src& src, dim3 grid, int nkb, int nb, int ld, const double2* becp, cudaStream_t s) {
+    k_proj_add<NT, GT, Src><<<grid, kWarps * 32, 0, s>>>(src, nkb, nb, ld, becp);
     note_launch();
     B200_CUDA(cudaGetLastError());
+}
+template <int NT, typename Src>
+void add_launch(const Src& src, int nk, int nkb, int nb, int ld, int npw_max, const double2* becp, cudaStream_t s) {
+    // 16 plane waves a warp, or 8 (a seventh more loads a product) where that leaves less of a last wave of three CTAs a
+    // SM idle
+    const int btiles = ceil_div(nb, 8 * NT);
+    auto grid = [&](int gt) { return dim3(ceil_div(npw_max, 8 * gt * kWarps), btiles, nk); };
+    auto waves = [&](int gt) { return (long(grid(gt).x) * btiles * nk + 443) / 444; };
+    if (double(waves(1)) * 1.15 < 2.0 * double(waves(2))) add_run<NT, 1>(src, grid(1), nkb, nb, ld, becp, s);
+    else add_run<NT, 2>(src, grid(2), nkb, nb, ld, becp, s);
 }
 
 // f(source of the k-points): by value, one or up to kMaxProjBatch
@@ -275,20 +284,39 @@ int npw_most(const ProjEntry* e, int nk) {
 
 }  // namespace
 
+// 8-band tiles a warp takes at a time, 1 to 4: the fewest padded bands, then the largest tile
+static int band_tiles(int nb) {
+    int best = 4, pad = 1 << 30;
+    for (int nt = 4; nt >= 1; --nt) {
+        const int p = ceil_div(nb, 8 * nt) * nt;
+        if (p < pad) {
+            pad = p;
+            best = nt;
+        }
+    }
+    return best;
+}
+
 void proj_becp(const ProjEntry* e, int nk, int nkb, int nb, int ld, double2* becp, ProjWorkspace& w, cudaStream_t s) {
     const int npw = npw_most(e, nk);
     with_source(e, nk, [&](const auto& src) {
-        if (nb <= 8) becp_launch<4, 1>(src, nk, nkb, nb, ld, npw, becp, w, s);
-        else if (nb <= 16) becp_launch<4, 2>(src, nk, nkb, nb, ld, npw, becp, w, s);
-        else becp_launch<2, 4>(src, nk, nkb, nb, ld, npw, becp, w, s);
+        switch (band_tiles(nb)) {
+            case 1: becp_launch<4, 1>(src, nk, nkb, nb, ld, npw, becp, w, s); break;
+            case 2: becp_launch<4, 2>(src, nk, nkb, nb, ld, npw, becp, w, s); break;
+            case 3: becp_launch<3, 3>(src, nk, nkb, nb, ld, npw, becp, w, s); break;
+            default: becp_launch<2, 4>(src, nk, nkb, nb, ld, npw, becp, w, s); break;
+        }
     });
 }
 void proj_add(const ProjEntry* e, int nk, int nkb, int nb, int ld, const double2* becp, cudaStream_t s) {
     const int npw = npw_most(e, nk);
     with_source(e, nk, [&](const auto& src) {
-        if (nb <= 8) add_launch<1>(src, nk, nkb, nb, ld, npw, becp, s);
-        else if (nb <= 16) add_launch<2>(src, nk, nkb, nb, ld, npw, becp, s);
-        else add_launch<4>(src, nk, nkb, nb, ld, npw, becp, s);
+        switch (band_tiles(nb)) {
+            case 1: add_launch<1>(src, nk, nkb, nb, ld, npw, becp, s); break;
+            case 2: add_launch<2>(src, nk, nkb, nb, ld, npw, becp, s); break;
+            case 3: add_launch<3>(src, nk, nkb, nb, ld, npw, becp, s); break;
+            default: add_launch<4>(src, nk, nkb, nb, ld, npw, becp, s); break;
+        }
     });
 }
 
@@ -297,5 +325,10 @@ void proj_add(const ProjEntry* e, int nk, int nkb, int nb, int ld, const double2
 // bands 28 / 28, 24 bands 35 / 53.  A batch saves the library's calls for every k-point: 64 x (64 x 3000), 32 bands,
 // 1.18 ms against 0.36.
 bool proj_small(int nkb, int nb, int npw, int nk) { return double(nkb) * nb * npw <= (nk > 1 ? 2e7 : 3e6); }
+// Against the int8 emulation, whose residues and recombination cost 39 ps a plane wave and band whatever the number of
+// projectors: 128 projectors x 9240, 61 bands 150 us of kernels against 81; 256 x 11 989, 64 bands 186 / 179; 256 x
+// 25 810, 64 bands 291 / 360 (these before the last waves were filled: now about a fifth less); 384 x 17 957, 48
+// bands 248 / 305.
+bool proj_beats_int8(int nkb, int nb, int npw) { return double(nkb) * nb * npw <= 2.5e8; }
 
 }  // namespace b200

@@ -27,5 +27,7 @@ void proj_becp(const ProjEntry* e, int nk, int nkb, int nb, int ld, double2* bec
 void proj_add(const ProjEntry* e, int nk, int nkb, int nb, int ld, const double2* becp, cudaStream_t s);
 // where these beat a library GEMM per product and k-point
 bool proj_small(int nkb, int nb, int npw, int nk);
+// where these beat the int8 emulation (gemm_oz.cu)
+bool proj_beats_int8(int nkb, int nb, int npw);
 
 }  // namespace b200
