@@ -1,6 +1,8 @@
-// sm_100a kernels for the G-sphere <-> r-box transforms and the fused local H|psi>.
+// sm_100a kernels for the G-sphere <-> r-box transforms and the fused local H|psi> of any 2-, 3-, 5-smooth grid: the
+// host maps, and the Stockham kernels for the grids that the line transforms (plane_g.cuh, box_lines.cu) do not cover
+// (an edge without two of their factors, a plane too large for shared memory).
 //
-// Fused local H|psi> (the hot path, replaces the per-band loop of
+// Fused local H|psi> (replaces the per-band loop of
 // Veff::act + Ekinetic::act in ABACUS, veff_pw.cpp:38-109, ekinetic_pw.cpp:34-50):
 //   1. k_zpass_inv : sphere scatter + inverse z FFT of a tile of sticks, written
 //                    plane-major into the stick buffer;
@@ -143,7 +145,6 @@ void PWGrid::ensure_device() {
     st_y.upload(h_sy.data(), nst);
     st_ixy.upload(h_sixy.data(), nst);
     xpos.upload(h_xpos.data(), nxc);
-    smap.upload(h_smap.data(), h_smap.size());
     if (lines.ok) cdesc.upload(h_cdesc.data(), h_cdesc.size());
     const size_t L = size_t(basis.npwk_max);
     for (int ik = 0; ik < basis.nks; ++ik) {

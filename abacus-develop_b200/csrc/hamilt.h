@@ -39,7 +39,7 @@ struct NonlocalK {
     bool nc_folded = false;
 };
 
-// Scratch of one H|psi> caller: stick buffer, becp, the padded-psi stage, a cuBLAS handle and the
+// Scratch of one H|psi> caller: stick buffer, becp, a cuBLAS handle and the
 // tensor-core GEMM workspace.  Callers that run H|psi> concurrently (different streams or threads) each
 // own one; the Hamiltonian itself is read-only after set-up.
 struct HpsiWork {

@@ -64,7 +64,6 @@ struct PlaneMapView {
     const int* xc;    // per stick: compact x-column index
     const int* sy;    // per stick: y
     const int* xpos;  // per compact column: x
-    const int* smap;  // per compact column c and y < ny: the stick at (xpos[c], y), or -1 (nxc x ny)
     // line transforms: the sticks of column c are those of y in [0, cd.y) and [cd.z, cd.w), from stick cd.x on;
     // the occupied x are [0, xm) and [xh, nx), x >= xh in column x - xoff
     const int4* cd;
@@ -93,8 +92,9 @@ struct PWGrid {
     PWBasisK basis;
     int nx = 0, ny = 0, nz = 0, nst = 0, nxc = 0;
     FftAxis ax, ay, az;
-    DeviceArray<int> st_xc, st_y, xpos, st_ixy, smap;
-    std::vector<int> h_xpos, h_xc, h_sy, h_sixy, h_smap;
+    DeviceArray<int> st_xc, st_y, xpos, st_ixy;
+    std::vector<int> h_xpos, h_xc, h_sy, h_sixy;
+    std::vector<int> h_smap;  // per compact column c and y < ny: the stick at (xpos[c], y), or -1 (nxc x ny)
     std::vector<KMap> kmaps;
     LinePlan lines;
     std::vector<int4> h_cdesc;
@@ -110,8 +110,7 @@ struct PWGrid {
         return StickMapView{nst, nz, k.gofs.ptr, k.gpk.ptr, k.glist.ptr, k.sd.ptr};
     }
     PlaneMapView plane_view() const {
-        return PlaneMapView{nst,      nxc,        st_xc.ptr, st_y.ptr, xpos.ptr,
-                            smap.ptr, cdesc.ptr, lines.xm,  lines.xh, lines.xoff};
+        return PlaneMapView{nst, nxc, st_xc.ptr, st_y.ptr, xpos.ptr, cdesc.ptr, lines.xm, lines.xh, lines.xoff};
     }
     long nxyz() const { return long(nx) * ny * nz; }
 };
