@@ -19,11 +19,11 @@
 //
 // What bounds the plane pass: latency at the 12 to 16 warps an SM's registers hold (128 to 168 a thread: a line's
 // R1 complex values, R2 - 1 twiddles, R2 values of V_eff).  Every point crosses shared memory eight times (128 bytes,
-// one cycle a point and SM): at 96^2 in FP64 that is 0.49 ms of 1.17 ms per 160 bands, and the FP64 pipe a third.
+// one cycle a point and SM): at 96^2 in FP64 that is 0.49 ms of 1.11 ms per 160 bands, and the FP64 pipe is 46 % busy.
 // Before it, edges without 32 as a factor ran one warp a line with up to six passes through shared memory, or the
 // Stockham kernels with a block barrier a pass.  FP64, B200, plane pass alone: 36^2 (2048 bands of 36 planes) 4.03 ->
-// 0.67 ms, 45^2 (61 x 90) 562 -> 88 us, 72 x 36 (120 x 108) 1966 -> 290 us; with its z passes the k batch's local
-// part went from 4.64 to 0.91 ms.  A compiled line takes half the time of a run-time one (36^2 1.36 ms, 45^2 144 us).
+// 0.67 ms, 45^2 (61 x 90) 562 -> 82 us, 72 x 36 (120 x 108) 1966 -> 284 us; with its z passes the k batch's local
+// part went from 4.64 to 0.87 ms.  A compiled line takes half the time of a run-time one (36^2 1.36 ms, 45^2 144 us).
 #pragma once
 #include "line_dft.cuh"
 #include "pw_grid.h"
