@@ -185,10 +185,9 @@ __global__ void __launch_bounds__(kBoxThreads) k_box_lines_x(PlaneMapView pm, Li
 
 namespace {
 
-template <typename K, typename... A>
-void box_launch(K kern, dim3 grid, size_t smem, cudaStream_t s, A... a) {
-    line::set_smem(kern, smem);
-    kern<<<grid, line::kBoxThreads, smem, s>>>(a...);
+template <auto Kernel, typename... A> void box_launch(dim3 grid, size_t smem, cudaStream_t s, A... a) {
+    allow_smem<Kernel>(smem);
+    Kernel<<<grid, line::kBoxThreads, smem, s>>>(a...);
     note_launch();
     B200_CUDA(cudaGetLastError());
 }
@@ -205,15 +204,15 @@ void box_both(const PWGrid& g, int ik, bool inverse, const T* in, T* out, T* aux
     const T *rx = line::roots_of<T>(g.ax), *ry = line::roots_of<T>(g.ay), *rz = line::roots_of<T>(g.az);
     const PlaneMapView pm = g.plane_view();
     if (inverse) {
-        box_launch(line::k_box_lines_z<T, R, RMAX, +1>, gz, sz, s, g.stick_view(ik), z, rz, in, sticks, 0, R(1));
-        box_launch(line::k_box_lines_y<T, RMAX, +1>, gy, sy, s, pm, y, g.nz, ry, (const T*)sticks, cols);
-        box_launch(line::k_box_lines_x<T, R, RMAX, +1>, gx, sx, s, pm, x, g.ny, g.nz, rx, (const T*)cols, out, add, R(factor));
+        box_launch<line::k_box_lines_z<T, R, RMAX, +1>>(gz, sz, s, g.stick_view(ik), z, rz, in, sticks, 0, R(1));
+        box_launch<line::k_box_lines_y<T, RMAX, +1>>(gy, sy, s, pm, y, g.nz, ry, (const T*)sticks, cols);
+        box_launch<line::k_box_lines_x<T, R, RMAX, +1>>(gx, sx, s, pm, x, g.ny, g.nz, rx, (const T*)cols, out, add, R(factor));
     } else {
         // set_real_to_recip_output_op: out (+)= factor / nxyz * box (pw_op.cpp:46-66)
         const double scale = (add ? factor : 1.0) / double(g.nxyz());
-        box_launch(line::k_box_lines_x<T, R, RMAX, -1>, gx, sx, s, pm, x, g.ny, g.nz, rx, in, cols, 0, R(1));
-        box_launch(line::k_box_lines_y<T, RMAX, -1>, gy, sy, s, pm, y, g.nz, ry, (const T*)cols, sticks);
-        box_launch(line::k_box_lines_z<T, R, RMAX, -1>, gz, sz, s, g.stick_view(ik), z, rz, (const T*)sticks, out, add, R(scale));
+        box_launch<line::k_box_lines_x<T, R, RMAX, -1>>(gx, sx, s, pm, x, g.ny, g.nz, rx, in, cols, 0, R(1));
+        box_launch<line::k_box_lines_y<T, RMAX, -1>>(gy, sy, s, pm, y, g.nz, ry, (const T*)cols, sticks);
+        box_launch<line::k_box_lines_z<T, R, RMAX, -1>>(gz, sz, s, g.stick_view(ik), z, rz, (const T*)sticks, out, add, R(scale));
     }
 }
 

@@ -4,6 +4,7 @@
 
 #include <cstddef>
 #include <cstdio>
+#include <mutex>
 #include <stdexcept>
 #include <string>
 
@@ -89,6 +90,22 @@ template <typename T> struct DeviceArray {
         if (count) B200_CUDA(cudaMemcpyAsync(ptr, host, count * sizeof(T), cudaMemcpyHostToDevice, s));
     }
 };
+
+// Before a launch of Kernel (without static shared memory) with `bytes` of dynamic shared memory: above the 48 KB that
+// need no leave, raises the kernel's limit to the card's, 227 KB, once per kernel and device.  The limit belongs to the
+// kernel, not to a launch: one that followed the launches' sizes would be lowered by a thread with a small launch
+// between another thread's raise and its launch.
+constexpr size_t kSmemMax = 227 * 1024;
+template <auto Kernel> void allow_smem(size_t bytes) {
+    if (bytes <= 48 * 1024) return;
+    constexpr int kDevices = 64;
+    static std::once_flag done[kDevices];
+    int dev = 0;
+    B200_CUDA(cudaGetDevice(&dev));
+    auto set = [] { B200_CUDA(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemMax))); };
+    if (dev < kDevices) std::call_once(done[dev], set);
+    else set();
+}
 
 inline int ceil_div(long a, long b) { return int((a + b - 1) / b); }
 

@@ -524,10 +524,6 @@ template <typename T> const T* tw_of(const FftAxis& a);
 template <> const double2* tw_of<double2>(const FftAxis& a) { return a.tw64.ptr; }
 template <> const float2* tw_of<float2>(const FftAxis& a) { return a.tw32.ptr; }
 
-template <typename K> static void set_smem(K kernel, size_t bytes) {
-    if (bytes > 48 * 1024) B200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
-}
-
 template <typename T, typename R>
 void launch_hpsi_local(const PWGrid& g, int ik, const R* veff_zyx, int nb, int ld, const T* psi, T* hpsi,
                        T* stickbuf, double tpiba2, int accumulate, cudaStream_t s) {
@@ -538,21 +534,21 @@ void launch_hpsi_local(const PWGrid& g, int ik, const R* veff_zyx, int nb, int l
     if (launch_hpsi_local_lines<T, R>(g, ik, veff_zyx, nb, ld, psi, hpsi, stickbuf, tpiba2, accumulate, s)) return;
     const size_t zs = zpass_smem(g, sizeof(T));
     const size_t ps = plane_smem(g, sizeof(T));
-    B200_CHECK(ps <= 227 * 1024, kCapacityError, "plane pass does not fit in shared memory for this grid");
+    B200_CHECK(ps <= kSmemMax, kCapacityError, "plane pass does not fit in shared memory for this grid");
     const StickMapView sm = g.stick_view(ik);
     const dim3 gz(ceil_div(g.nst, kStickTile), nb);
-    set_smem(k_zpass_inv<T>, zs);
+    allow_smem<k_zpass_inv<T>>(zs);
     k_zpass_inv<T><<<gz, 256, zs, s>>>(sm, g.az.plan, tw_of<T>(g.az), psi, ld, stickbuf);
     note_launch();
     B200_CUDA(cudaGetLastError());
-    set_smem(k_plane<T, R>, ps);
+    allow_smem<k_plane<T, R>>(ps);
     k_plane<T, R><<<dim3(nb, g.nz), 512, ps, s>>>(g.plane_view(), g.nx, g.ny, g.nz, g.ax.plan, g.ay.plan, tw_of<T>(g.ax),
                                                   tw_of<T>(g.ay), veff_zyx, stickbuf);
     note_launch();
     B200_CUDA(cudaGetLastError());
     const KMap& km = g.kmaps[ik];
     const R* gk2 = std::is_same<R, double>::value ? (const R*)km.gk2.ptr : (const R*)km.gk2f.ptr;
-    set_smem(k_zpass_fwd<T, R>, zs);
+    allow_smem<k_zpass_fwd<T, R>>(zs);
     k_zpass_fwd<T, R><<<gz, 256, zs, s>>>(sm, g.az.plan, tw_of<T>(g.az), stickbuf, psi, hpsi, ld, km.npw, gk2, R(tpiba2),
                                           R(1.0 / double(g.nxyz())), accumulate);
     note_launch();
@@ -567,26 +563,26 @@ void launch_hpsi_local_nc(const PWGrid& g, int ik, const R* veff4_zyx, int ncols
     if (launch_hpsi_local_nc_lines<T, R>(g, ik, veff4_zyx, ncols, ld, psi, hpsi, stickbuf, tpiba2, s)) return;
     const size_t zs = zpass_smem(g, sizeof(T));
     const size_t ps = plane_smem(g, sizeof(T));
-    B200_CHECK(ps <= 227 * 1024, kCapacityError, "plane pass does not fit in shared memory for this grid");
+    B200_CHECK(ps <= kSmemMax, kCapacityError, "plane pass does not fit in shared memory for this grid");
     const StickMapView sm = g.stick_view(ik);
     const dim3 gz(ceil_div(g.nst, kStickTile), ncols);
-    set_smem(k_zpass_inv<T>, zs);
+    allow_smem<k_zpass_inv<T>>(zs);
     k_zpass_inv<T><<<gz, 256, zs, s>>>(sm, g.az.plan, tw_of<T>(g.az), psi, ld, stickbuf);
     note_launch();
     B200_CUDA(cudaGetLastError());
-    set_smem(k_plane_inv_r<T>, ps);
+    allow_smem<k_plane_inv_r<T>>(ps);
     k_plane_inv_r<T><<<dim3(ncols, g.nz), 512, ps, s>>>(g.plane_view(), g.nx, g.ny, g.nz, g.ax.plan, g.ay.plan,
                                                        tw_of<T>(g.ax), tw_of<T>(g.ay), stickbuf, rbuf);
     note_launch();
     B200_CUDA(cudaGetLastError());
-    set_smem(k_plane_fwd_nc<T, R>, ps);
+    allow_smem<k_plane_fwd_nc<T, R>>(ps);
     k_plane_fwd_nc<T, R><<<dim3(ncols, g.nz), 512, ps, s>>>(g.plane_view(), g.nx, g.ny, g.nz, g.ax.plan, g.ay.plan,
                                                            tw_of<T>(g.ax), tw_of<T>(g.ay), veff4_zyx, rbuf, stickbuf);
     note_launch();
     B200_CUDA(cudaGetLastError());
     const KMap& km = g.kmaps[ik];
     const R* gk2 = std::is_same<R, double>::value ? (const R*)km.gk2.ptr : (const R*)km.gk2f.ptr;
-    set_smem(k_zpass_fwd<T, R>, zs);
+    allow_smem<k_zpass_fwd<T, R>>(zs);
     k_zpass_fwd<T, R><<<gz, 256, zs, s>>>(sm, g.az.plan, tw_of<T>(g.az), stickbuf, psi, hpsi, ld, km.npw, gk2, R(tpiba2),
                                           R(1.0 / double(g.nxyz())), 0);
     note_launch();
@@ -600,19 +596,19 @@ void launch_recip_to_real(const PWGrid& g, int ik, const T* in, T* out, T* aux, 
     const size_t N = size_t(g.nxyz());
     B200_CUDA(cudaMemsetAsync(aux, 0, N * sizeof(T), s));
     const size_t zs = zpass_smem(g, sizeof(T));
-    set_smem(k_box_zinv<T>, zs);
+    allow_smem<k_box_zinv<T>>(zs);
     k_box_zinv<T><<<ceil_div(g.nst, kStickTile), 256, zs, s>>>(g.stick_view(ik), g.az.plan, tw_of<T>(g.az), g.st_ixy.ptr,
                                                                in, aux);
     note_launch();
     B200_CUDA(cudaGetLastError());
     const size_t ys = size_t(2) * kBoxTile * odd_ld(g.ny) * sizeof(T);
-    set_smem(k_box_y<T, +1>, ys);
+    allow_smem<k_box_y<T, +1>>(ys);
     k_box_y<T, +1><<<dim3(g.nxc, ceil_div(g.nz, kBoxTile)), 256, ys, s>>>(g.ay.plan, tw_of<T>(g.ay), g.xpos.ptr, g.ny,
                                                                           g.nz, aux);
     note_launch();
     B200_CUDA(cudaGetLastError());
     const size_t xsm = size_t(2) * kBoxTile * odd_ld(g.nx) * sizeof(T);
-    set_smem(k_box_x<T, R, +1>, xsm);
+    allow_smem<k_box_x<T, R, +1>>(xsm);
     k_box_x<T, R, +1><<<dim3(g.ny, ceil_div(g.nz, kBoxTile)), 256, xsm, s>>>(g.ax.plan, tw_of<T>(g.ax), g.nx, g.ny, g.nz,
                                                                              aux, out, add, R(factor));
     note_launch();
@@ -624,19 +620,19 @@ void launch_real_to_recip(const PWGrid& g, int ik, const T* in, T* out, T* aux, 
     if (launch_box_lines<T>(g, ik, false, in, out, aux, add, factor, s)) return;
     using R = typename RealOf<T>::type;
     const size_t xsm = size_t(2) * kBoxTile * odd_ld(g.nx) * sizeof(T);
-    set_smem(k_box_x<T, R, -1>, xsm);
+    allow_smem<k_box_x<T, R, -1>>(xsm);
     k_box_x<T, R, -1><<<dim3(g.ny, ceil_div(g.nz, kBoxTile)), 256, xsm, s>>>(g.ax.plan, tw_of<T>(g.ax), g.nx, g.ny, g.nz,
                                                                              in, aux, 0, R(1));
     note_launch();
     B200_CUDA(cudaGetLastError());
     const size_t ys = size_t(2) * kBoxTile * odd_ld(g.ny) * sizeof(T);
-    set_smem(k_box_y<T, -1>, ys);
+    allow_smem<k_box_y<T, -1>>(ys);
     k_box_y<T, -1><<<dim3(g.nxc, ceil_div(g.nz, kBoxTile)), 256, ys, s>>>(g.ay.plan, tw_of<T>(g.ay), g.xpos.ptr, g.ny,
                                                                           g.nz, aux);
     note_launch();
     B200_CUDA(cudaGetLastError());
     const size_t zs = zpass_smem(g, sizeof(T));
-    set_smem(k_box_zfwd<T, R>, zs);
+    allow_smem<k_box_zfwd<T, R>>(zs);
     // set_real_to_recip_output_op: out (+)= factor / nxyz * box (pw_op.cpp:46-66)
     const double scale = (add ? factor : 1.0) / double(g.nxyz());
     k_box_zfwd<T, R><<<ceil_div(g.nst, kStickTile), 256, zs, s>>>(g.stick_view(ik), g.az.plan, tw_of<T>(g.az),

@@ -7,8 +7,6 @@ namespace b200 {
 
 namespace {
 
-constexpr size_t kSmemMax = 227 * 1024;
-
 constexpr int kSMs = 148;
 // the class of a run-time r1 (RMAX of the kernels)
 int rmax_of(int r) { return r <= 10 ? 10 : r <= 16 ? 16 : 25; }

@@ -17,14 +17,11 @@ template <typename T> const T* roots_of(const FftAxis& a) {
     if constexpr (sizeof(T) == 16) return a.rt64.ptr;
     else return a.rt32.ptr;
 }
-template <typename K> void set_smem(K kernel, size_t bytes) {
-    if (bytes > 48 * 1024) B200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
-}
 
 template <typename T, typename R, int RMAX, int NPOL, typename GX, typename GY>
 void plane_launch(const PWGrid& g, const PlaneShape& sh, int nplanes, GX gx, GY gy, const R* v, T* sb, cudaStream_t s) {
-    auto kern = k_plane_g<T, R, RMAX, NPOL, plane_threads(sizeof(T), RMAX), GX, GY>;
-    set_smem(kern, sh.smem);
+    constexpr auto kern = k_plane_g<T, R, RMAX, NPOL, plane_threads(sizeof(T), RMAX), GX, GY>;
+    allow_smem<kern>(sh.smem);
     kern<<<dim3(nplanes, g.nz), sh.nw * 32, sh.smem, s>>>(g.plane_view(), gx, gy, sh.L, g.nz, roots_of<T>(g.ax),
                                                           roots_of<T>(g.ay), v, size_t(g.nxyz()), sb);
     note_launch();
@@ -63,9 +60,9 @@ template <typename T, typename R> struct RhoArgs {
 };
 template <typename T, typename R, int RMAX, typename GX, typename GY>
 void rho_launch(const PWGrid& g, GX gx, GY gy, const RhoArgs<T, R>& a) {
-    auto kern = k_rho_g<T, R, RMAX, plane_threads(sizeof(T), RMAX), GX, GY>;
+    constexpr auto kern = k_rho_g<T, R, RMAX, plane_threads(sizeof(T), RMAX), GX, GY>;
     const PlaneShape& sh = a.shape.plane;
-    set_smem(kern, sh.smem);
+    allow_smem<kern>(sh.smem);
     kern<<<dim3(g.nz, a.shape.nsplit), sh.nw * 32, sh.smem, a.s>>>(g.plane_view(), gx, gy, sh.L, g.nz, roots_of<T>(g.ax),
                                                                   roots_of<T>(g.ay), a.sb, a.nbc, a.w, a.shape.nsplit,
                                                                   a.shape.sums, a.ws, a.first);
@@ -107,12 +104,12 @@ void z_launch(const PWGrid& g, GZ gz, const ZArgs<T, Src>& a) {
     const size_t smem = size_t(TS) * gz.ld * sizeof(T);
     const dim3 grid(ceil_div(g.nst, TS), a.nbc, a.nk);
     if (a.inv) {
-        auto kern = k_zinv_g<T, RMAX, TS, ZT, Src, GZ>;
-        set_smem(kern, smem);
+        constexpr auto kern = k_zinv_g<T, RMAX, TS, ZT, Src, GZ>;
+        allow_smem<kern>(smem);
         kern<<<grid, ZT, smem, a.s>>>(a.src, gz, a.b0, a.nbc, roots_of<T>(g.az), a.sb);
     } else {
-        auto kern = k_zfwd_g<T, R, RMAX, TS, ZT, Src, GZ>;
-        set_smem(kern, smem);
+        constexpr auto kern = k_zfwd_g<T, R, RMAX, TS, ZT, Src, GZ>;
+        allow_smem<kern>(smem);
         kern<<<grid, ZT, smem, a.s>>>(a.src, gz, a.b0, a.nbc, roots_of<T>(g.az), a.sb, R(a.tpiba2),
                                        R(1.0 / double(g.nxyz())), a.accumulate);
     }

@@ -1,0 +1,89 @@
+"""Several host threads on one basis: their launches share kernels, whose state (the limit of dynamic shared memory) no
+thread may change under another.  At 96 x 96 the plane pass's launch shape, and with it the shared memory, changes with
+the band count, so threads with different band counts meet each other's sizes at every call."""
+from __future__ import annotations
+
+import dataclasses
+import threading
+
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+def _run_threads(jobs):
+    errors = []
+
+    def guard(job):
+        try:
+            job()
+        except BaseException as e:  # noqa: BLE001 - reported by the caller
+            errors.append(e)
+    threads = [threading.Thread(target=guard, args=(j,)) for j in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors[0]
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+def test_local_pass_with_different_band_counts(pkg, prec):
+    """Three handles of one basis, a thread and a stream each, bands 1 to 8 in different orders: bit for bit the
+    results of the same calls alone."""
+    P = pkg.pwdft
+    n = 96
+    b = P.PWBasisK(0.28, np.diag([float(n)] * 3), 30.0, np.array([[0.125, -0.375, 0.375]]), grid=(n, n, n))
+    rng = np.random.default_rng(4)
+    npw, ld = int(b.npwk[0]), int(b.npwk_max)
+    ct = torch.complex128 if prec == "fp64" else torch.complex64
+    psi = torch.from_numpy(rng.standard_normal((8, ld)) + 1j * rng.standard_normal((8, ld))).to("cuda", ct)
+    veff = torch.from_numpy(rng.uniform(-2.0, 0.5, size=b.nxyz)).cuda()
+    hs = [P.HamiltPW(b, P.PREC_FP64 if prec == "fp64" else P.PREC_MIXED) for _ in range(3)]
+    for h in hs:
+        h.set_veff(veff)
+    want = {}
+    for nb in (1, 2, 3, 4, 5, 7, 8):
+        want[nb] = torch.zeros_like(psi[:nb])
+        hs[0].hpsi_part(0, psi, want[nb], nb, ld, 1)
+    torch.cuda.synchronize()
+
+    def job(h, counts):
+        def run():
+            s = torch.cuda.Stream()
+            with torch.cuda.stream(s):
+                out = torch.zeros_like(psi)
+                for i in range(400):
+                    nb = counts[i % len(counts)]
+                    h.hpsi_part(0, psi, out, nb, ld, 1)
+                    if i % 25 < len(counts):
+                        assert torch.equal(out[:nb], want[nb]), (i, nb)
+                s.synchronize()
+        return run
+    _run_threads([job(hs[0], (1, 5, 2)), job(hs[1], (8, 1, 4)), job(hs[2], (3, 7))])
+
+
+def test_concurrent_mixed_solves_at_96(pkg):
+    """Four workers on one Hamiltonian, so that their unconverged bands differ: each k-point's eigenvalues and iteration
+    count of its solve alone."""
+    P = pkg.pwdft
+    spec = dataclasses.replace(pkg.synth.config(0), grid=(96, 96, 96))
+    wl = P.build_workload(spec, kpts=pkg.synth.mp_grid(2, True)[:4])
+    h = P.device_hamilt(wl, P.PREC_FP64)
+    nband, ld = 6, wl.basis.npwk_max
+    iks = list(range(4))
+    pcs = [P.precondition_d(wl.basis, ik) for ik in iks]
+    start = [torch.from_numpy(wl.psi0_h[ik][:nband].reshape(-1).copy()).cuda() for ik in iks]
+    alone, its_alone = [], []
+    for ik in iks:
+        dav = P.DiagoDavid(pcs[ik], nband, int(wl.basis.npwk[ik]), 4, P.PREC_MIXED)
+        e = np.zeros(nband)
+        its_alone.append(dav.diag_hamilt(h, ik, ld, start[ik].clone(), e, 1e-9, 100))
+        alone.append(e)
+    for _ in range(5):
+        eig, its = h.solve_kpoints(iks, pcs, [x.clone() for x in start], ld, nband, 1e-9, 100, precision=P.PREC_MIXED,
+                                   nworkers=4)
+        assert np.max(np.abs(np.asarray(eig) - np.asarray(alone))) < 1e-9
+        assert list(its) == its_alone
