@@ -33,14 +33,15 @@ template <bool CONJ> __device__ __forceinline__ void zmma(double (&re)[2], doubl
 
 struct OneProj {
     ProjEntry e;
-    __device__ __forceinline__ const ProjEntry& get(int) const { return e; }
+    __host__ __device__ __forceinline__ const ProjEntry& get(int) const { return e; }
 };
 struct ManyProj {
     ProjEntry e[kMaxProjBatch];
-    __device__ __forceinline__ const ProjEntry& get(int q) const { return e[q]; }
+    __host__ __device__ __forceinline__ const ProjEntry& get(int q) const { return e[q]; }
 };
 
 constexpr int kWarps = 4;
+constexpr int kWave = 3 * 148;  // CTAs of one wave at three a SM
 
 // grid: x = projector tile + slice * tiles, y = band tile, z = k-point
 template <int JT, int NT, typename Src>
@@ -226,6 +227,18 @@ __global__ void __launch_bounds__(kWarps * 32) k_proj_add(Src src, int nkb, int 
             }
 }
 
+int slices_most(int npw) { return std::max(1, int(std::sqrt(npw / 8.0))); }
+// What becp_launch may need of partial sums for a call of this size or any smaller one.  A call's own need is not
+// monotone in its bands (8 k-points x 64 projectors: 248 832 values at 24 bands, 212 992 at 32), and an array of just
+// that size would be freed by a smaller call under a captured graph that holds its address.  Tiles are at most 4 x 4
+// blocks of 8 x 8 and 9 in all, and several slices mean tiles * slices <= kWave.
+template <typename Src> size_t part_bound(const Src& src, int nk, int nkb, int nb) {
+    int npwx = 0;
+    for (int q = 0; q < nk; ++q) npwx = std::max(npwx, src.get(q).npwx);
+    const size_t blocks = size_t(nk) * (ceil_div(nkb, 8) + 3) * (ceil_div(nb, 8) + 3);
+    return std::min(blocks * slices_most(npwx), size_t(kWave) * 9) * 64;
+}
+
 template <int JT, int NT, typename Src>
 void becp_launch(const Src& src, int nk, int nkb, int nb, int ld, int npw_max, double2* becp, ProjWorkspace& w,
                  cudaStream_t s) {
@@ -233,11 +246,12 @@ void becp_launch(const Src& src, int nk, int nkb, int nb, int ld, int npw_max, d
     const long tiles = long(nk) * jtiles * btiles;
     // slices of the plane waves: one wave of three CTAs a SM; a step of a warp (4 plane waves) costs about twice what the
     // last CTA takes to add a slice, so a single tile's time is least near sqrt(steps / 2) slices
-    const int slices = int(std::max(1.0, std::min(double(std::max<long>(1, 444 / tiles)), std::sqrt(npw_max / 8.0))));
+    const int slices = std::min(int(std::max<long>(1, kWave / tiles)), slices_most(npw_max));
+    static_assert(JT <= 4 && NT <= 4 && JT * NT <= 9, "part_bound");
     if (slices > 1) {
-        w.part.resize(size_t(tiles) * slices * JT * NT * 64);
-        if (w.count.n < size_t(tiles)) {
-            w.count.resize(size_t(tiles));
+        w.part.resize(part_bound(src, nk, nkb, nb));
+        if (!w.count.ptr) {
+            w.count.resize(kWave);
             B200_CUDA(cudaMemsetAsync(w.count.ptr, 0, w.count.n * sizeof(unsigned), s));
         }
     }
@@ -258,7 +272,7 @@ void add_launch(const Src& src, int nk, int nkb, int nb, int ld, int npw_max, co
     // SM idle
     const int btiles = ceil_div(nb, 8 * NT);
     auto grid = [&](int gt) { return dim3(ceil_div(npw_max, 8 * gt * kWarps), btiles, nk); };
-    auto waves = [&](int gt) { return (long(grid(gt).x) * btiles * nk + 443) / 444; };
+    auto waves = [&](int gt) { return (long(grid(gt).x) * btiles * nk + kWave - 1) / kWave; };
     if (double(waves(1)) * 1.15 < 2.0 * double(waves(2))) add_run<NT, 1>(src, grid(1), nkb, nb, ld, becp, s);
     else add_run<NT, 2>(src, grid(2), nkb, nb, ld, becp, s);
 }

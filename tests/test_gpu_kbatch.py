@@ -138,6 +138,33 @@ def test_graph_replay_equals_direct(pkg, mp444):
     del g
 
 
+def test_graph_replay_after_a_smaller_eager_call(pkg, mp444):
+    """A call with fewer bands may cut the projector products into more slices (8 k-points x 64 projectors: 248 832
+    partial sums at 24 bands, 212 992 at 32) and must leave the scratch of a captured batch where it is."""
+    spec, wl = mp444
+    P = pkg.pwdft
+    h = P.device_hamilt(wl, P.PREC_FP64)
+    nb, ld, iks = 32, wl.basis.npwk_max, list(range(8))
+    psis = _psis(wl, nb, np.complex128)
+    outs = [torch.zeros_like(x) for x in psis]
+    s = torch.cuda.Stream()
+    g = h.capture_hpsi_kbatch(iks, psis, outs, nb, ld, stream=s)
+    s.synchronize()
+    want = [x.clone() for x in outs]
+    small = [torch.zeros_like(x) for x in psis]
+    for fewer in (24, 17, 9, 1):
+        h.hpsi_kbatch(iks, psis, small, fewer, ld)
+    torch.cuda.synchronize()
+    for x in outs:
+        x.zero_()
+    torch.cuda.synchronize()
+    g.launch(s)
+    s.synchronize()
+    for q in iks:
+        assert torch.equal(outs[q], want[q])
+    del g
+
+
 def test_autotune_keeps_result(pkg, mp444):
     spec, wl = mp444
     P = pkg.pwdft
