@@ -19,6 +19,8 @@
 #include "capi_handles.h"
 
 struct b200_graph {
+    // the addresses in the graph: a scratch that calls on the handle could reallocate would leave it dangling
+    b200::HpsiWork work;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     ~b200_graph() {
@@ -32,14 +34,14 @@ namespace {
 using b200::guarded;
 
 void kbatch_call(b200_hamilt* h, int nk, const int* iks, int spin, int nb, int ld, void* const* psi, void* const* hpsi,
-                 cudaStream_t s) {
+                 cudaStream_t s, b200::HpsiWork* w = nullptr) {
     B200_CHECK(h && iks && psi && hpsi, b200::kInvalidArgument, "NULL argument");
     if (h->h->precision == B200_PREC_FP64)
         h->h->hpsi_kbatch<double2>(nk, iks, spin, nb, ld, reinterpret_cast<const double2* const*>(psi),
-                                   reinterpret_cast<double2* const*>(hpsi), s);
+                                   reinterpret_cast<double2* const*>(hpsi), s, w);
     else
         h->h->hpsi_kbatch<float2>(nk, iks, spin, nb, ld, reinterpret_cast<const float2* const*>(psi),
-                                  reinterpret_cast<float2* const*>(hpsi), s);
+                                  reinterpret_cast<float2* const*>(hpsi), s, w);
 }
 
 }  // namespace
@@ -58,12 +60,12 @@ int b200_graph_capture_hpsi_kbatch(b200_hamilt* h, int nk, const int* iks, int s
         cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
         B200_CHECK(s != nullptr, b200::kInvalidArgument, "capture needs a non-default stream");
         // one eager call first: every workspace is allocated and every kernel attribute set before capture
-        kbatch_call(h, nk, iks, spin, nbands, ld, psi_d, hpsi_d, s);
-        B200_CUDA(cudaStreamSynchronize(s));
         auto g = std::make_unique<b200_graph>();
+        kbatch_call(h, nk, iks, spin, nbands, ld, psi_d, hpsi_d, s, &g->work);
+        B200_CUDA(cudaStreamSynchronize(s));
         B200_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
         try {
-            kbatch_call(h, nk, iks, spin, nbands, ld, psi_d, hpsi_d, s);
+            kbatch_call(h, nk, iks, spin, nbands, ld, psi_d, hpsi_d, s, &g->work);
         } catch (...) {
             cudaGraph_t dead = nullptr;
             cudaStreamEndCapture(s, &dead);

@@ -213,8 +213,9 @@ int b200_hamilt_hpsi_kbatch(b200_hamilt* h, int nk, const int* iks, int spin, in
                             void* const* hpsi_d, void* stream);
 /* Captures b200_hamilt_hpsi_kbatch with these arguments into a CUDA graph (after one eager call that
  * allocates every workspace; the eager call's output is the same as a replay's).  stream must not be
- * the legacy default stream.  Replays read psi_d and write hpsi_d at the captured addresses.
- * No counterpart in the reference. */
+ * the legacy default stream.  Replays read psi_d and write hpsi_d at the captured addresses.  The graph owns
+ * its scratch (what one such call takes), so later calls on h may be of any size; V_eff and the projectors
+ * stay h's.  No counterpart in the reference. */
 int b200_graph_capture_hpsi_kbatch(b200_hamilt* h, int nk, const int* iks, int spin, int nbands, int ld,
                                    void* const* psi_d, void* const* hpsi_d, void* stream, b200_graph** out);
 int b200_graph_launch(b200_graph* g, void* stream);

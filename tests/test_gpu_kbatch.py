@@ -165,6 +165,36 @@ def test_graph_replay_after_a_smaller_eager_call(pkg, mp444):
     del g
 
 
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+def test_graph_replay_after_larger_eager_calls(pkg, mp444, prec):
+    """The graph owns its scratch: eager calls of more bands and k-points on the same handle, which take larger arrays,
+    and buffers allocated afterwards change nothing of a replay."""
+    spec, wl = mp444
+    P = pkg.pwdft
+    h = P.device_hamilt(wl, P.PREC_FP64 if prec == "fp64" else P.PREC_MIXED)
+    dt = np.complex128 if prec == "fp64" else np.complex64
+    nb, ld, iks = 3, wl.basis.npwk_max, [1, 4]
+    all_psis = _psis(wl, 32, dt)
+    psis = [all_psis[ik][:nb * ld].clone() for ik in iks]
+    outs = [torch.zeros_like(x) for x in psis]
+    s = torch.cuda.Stream()
+    g = h.capture_hpsi_kbatch(iks, psis, outs, nb, ld, stream=s)
+    s.synchronize()
+    want = [x.clone() for x in outs]
+    big = [torch.zeros_like(x) for x in all_psis]
+    h.hpsi_kbatch(range(8), all_psis, big, 32, ld)
+    h.hpsi(0, all_psis[0], big[0], 32, ld)
+    filler = [torch.full((1 << 20,), float("nan"), device="cuda") for _ in range(16)]
+    for x in outs:
+        x.zero_()
+    torch.cuda.synchronize()
+    g.launch(s)
+    s.synchronize()
+    for q in range(len(iks)):
+        assert torch.equal(outs[q], want[q])
+    del g, filler
+
+
 def test_autotune_keeps_result(pkg, mp444):
     spec, wl = mp444
     P = pkg.pwdft
