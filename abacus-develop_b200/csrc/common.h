@@ -91,11 +91,13 @@ template <typename T> struct DeviceArray {
     }
 };
 
+constexpr int kMaxGridY = 65535;         // CTAs along y or z of a launch
+constexpr size_t kSmemMax = 227 * 1024;  // dynamic shared memory of a CTA
+
 // Before a launch of Kernel (without static shared memory) with `bytes` of dynamic shared memory: above the 48 KB that
 // need no leave, raises the kernel's limit to the card's, 227 KB, once per kernel and device.  The limit belongs to the
 // kernel, not to a launch: one that followed the launches' sizes would be lowered by a thread with a small launch
 // between another thread's raise and its launch.
-constexpr size_t kSmemMax = 227 * 1024;
 template <auto Kernel> void allow_smem(size_t bytes) {
     if (bytes <= 48 * 1024) return;
     constexpr int kDevices = 64;

@@ -599,6 +599,7 @@ void Hamilt::hpsi_kbatch(int nk, const int* iks, int spin, int nb, int ld, const
     int chunk = chunk_override > 0 ? chunk_override : int(std::min<size_t>(nb, W.stick_bytes / (per_band * nk)));
     if (chunk < 1) chunk = 1;
     if (chunk > nb) chunk = nb;
+    if (chunk > kMaxGridY) chunk = kMaxGridY;  // the z passes put the bands on gridDim.y
     const R* veff = f64 ? (const R*)veff_zyx.ptr : (const R*)veff_zyxf.ptr;
     T* sb;
     if constexpr (f64) {

@@ -74,8 +74,8 @@ void hpsi_local_noalloc(b200::Hamilt& H, int ik, int nb, int ld, const T* psi, T
                    std::to_string(kNoAllocScratchBytes) + "-byte no-alloc scratch");
     if (nb == 0) return;
     T* sb = static_cast<T*>(noalloc_scratch_on_current_device());
-    // bands per launch: what the scratch holds, and at most 65535 (the launches put bands on gridDim.y)
-    const int chunk = int(std::min<size_t>(kNoAllocScratchBytes / per_band, 65535));
+    // bands per launch: what the scratch holds, and no more than gridDim.y takes
+    const int chunk = int(std::min<size_t>(kNoAllocScratchBytes / per_band, b200::kMaxGridY));
     const R* veff = H.veff_of<R>();
     for (int b0 = 0; b0 < nb; b0 += chunk) {
         const int nbc = nb - b0 < chunk ? nb - b0 : chunk;

@@ -100,7 +100,9 @@ void psi_to_rho(b200_pw_basis* b, b200::DeviceArray<T>& box, b200::DeviceArray<T
         b->rho_w.resize(size_t(nbands));
         B200_CUDA(cudaMemcpyAsync(b->rho_w.ptr, w1, size_t(nbands) * sizeof(double), cudaMemcpyHostToDevice, s));
         const size_t per_band = size_t(g.nz) * g.nst;
-        const int chunk = int(std::min<size_t>(nbands, std::max<size_t>(1, b200::kStickBytes / (per_band * sizeof(T)))));
+        // (the z pass puts the bands on gridDim.y)
+        const int chunk = int(std::min<size_t>(std::min(nbands, b200::kMaxGridY),
+                                               std::max<size_t>(1, b200::kStickBytes / (per_band * sizeof(T)))));
         sbuf.resize(size_t(chunk) * per_band);
         const b200::RhoShape shape = b200::rho_shape(g, sizeof(T), chunk);
         ws.resize(size_t(shape.nsplit) * size_t(g.nxyz()));

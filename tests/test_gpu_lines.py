@@ -86,6 +86,23 @@ def test_kbatch_on_lines_matches_oracle(pkg, grid, prec):
 
 
 @pytest.mark.gpu
+def test_kbatch_of_more_bands_than_a_launch_takes(pkg):
+    """12 x 12 x 12 in FP32: the stick buffer holds more bands than gridDim.y; 70 000 bands of seven vectors."""
+    torch = pytest.importorskip("torch")
+    P = pkg.pwdft
+    b, ref = _setup(pkg, (12, 12, 12))
+    veff, psi, ld = _inputs(b, 0, 7)
+    h = P.HamiltPW(b, P.PREC_MIXED)
+    h.set_veff(torch.from_numpy(veff).cuda())
+    pd = torch.from_numpy(psi).to("cuda", torch.complex64).repeat(10000, 1)
+    hd = torch.full_like(pd, 7.0)
+    h.hpsi_kbatch([0], [pd], [hd], len(pd), ld)
+    want = torch.from_numpy(_oracle(ref, 0, veff, psi, 7, ld).reshape(7, ld)).cuda()
+    diff = (hd.view(10000, 7, ld) - want).abs().max()
+    assert float(diff / want.abs().max()) < 2e-5
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("prec", [0, 1])
 @pytest.mark.parametrize("grid,nb", [((18, 18, 18), 3), ((36, 45, 20), 2), ((75, 75, 16), 1), ((90, 96, 25), 1)])
 def test_spinor_local_pass_matches_oracle(pkg, grid, nb, prec):

@@ -14,6 +14,23 @@ CASES = [((18, 18, 18), 1), ((20, 25, 32), 7), ((36, 36, 45), 33), ((72, 36, 50)
 
 
 @pytest.mark.gpu
+def test_more_bands_than_a_launch_takes(pkg):
+    """A 12 x 12 x 12 grid's stick buffer holds more bands than gridDim.y: seven bands, each 10 000 times."""
+    torch = pytest.importorskip("torch")
+    grid, nb, times = (12, 12, 12), 7, 10000
+    lat, k = np.diag(np.array(grid, dtype=float)), np.array([[0.125, -0.375, 0.375]])
+    b = pkg.pwdft.PWBasisK(0.28, lat, 30.0, k, grid=grid)
+    ref = PWBasisKRef(0.28, lat, 30.0, k, grid=grid)
+    rng = np.random.default_rng(8)
+    npw = int(b.npwk[0])
+    psi = rng.standard_normal((nb, npw)) + 1j * rng.standard_normal((nb, npw))
+    want = sum(np.abs(H.recip_to_real(ref, p, 0)) ** 2 for p in psi)
+    rho = torch.zeros(b.nxyz, dtype=torch.float64, device="cuda")
+    b.psi_to_rho(0, torch.from_numpy(psi).cuda().repeat(times, 1), nb * times, npw, np.full(nb * times, 1.0 / times), rho)
+    assert np.max(np.abs(rho.cpu().numpy() - want)) / np.max(want) < 1e-12
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("prec", [0, 1])
 @pytest.mark.parametrize("grid,nb", CASES)
 def test_rho_matches_oracle(pkg, grid, nb, prec):
