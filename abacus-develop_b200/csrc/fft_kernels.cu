@@ -83,8 +83,14 @@ void PWGrid::build(const PWBasisK& b) {
     on_device = false;
     B200_CHECK(nz < 1024, kInvalidArgument, "nz must be < 1024");
     ax.build(nx);
-    ay.build(ny);
-    az.build(nz);
+    for (auto [axis, n] : {std::pair<FftAxis*, int>{&ay, ny}, {&az, nz}}) {
+        if (n == nx) {  // the same plan and twiddles
+            axis->plan = ax.plan;
+            axis->h_tw64 = ax.h_tw64;
+        } else {
+            axis->build(n);
+        }
+    }
     std::vector<int> sx(nst);
     h_sy.assign(nst, 0);
     h_sixy.assign(nst, 0);

@@ -13,16 +13,23 @@ int rmax_of(int r) { return r <= 10 ? 10 : r <= 16 ? 16 : 25; }
 
 // instructions of the busiest of nw warps with L rows at a time, from the operation counts (x transforms one way
 // only and no V_eff for inverse_only)
-double warp_work(const LineGeom& x, const LineGeom& y, int ncols, int npol, int nw, int L, bool inverse_only) {
-    const int na = 32 / x.r2, nb = 32 / x.r1, nya = 32 / y.r2, nyb = 32 / y.r1, ways = inverse_only ? 1 : 2;
-    const double ca = ways * line::dft_ops(x.r1) + 5 * ways * x.r1 + 40;
-    const double cb = npol * (ways * line::dft_ops(x.r2) + 6 * ways * (x.r2 - 1) + 10 * ways * x.r2);
-    const double cya = ways * line::dft_ops(y.r1) + 15 * ways * y.r1 + 40;
-    const double cyb = ways * line::dft_ops(y.r2) + 6 * ways * y.r2 + 10 * ways * y.r2;
-    const int groups = ceil_div(ceil_div(y.n, L), nw), cper = ceil_div(ncols, nw);
-    return groups * (ceil_div(npol * L, na) * ca + ceil_div(L, nb) * cb) + ceil_div(cper, nya) * cya +
-           ceil_div(cper, nyb) * cyb;
-}
+struct WarpWork {
+    int ny, ncols, npol, na, nb, nya, nyb;
+    double ca, cb, cya, cyb;
+    WarpWork(const LineGeom& x, const LineGeom& y, int ncols_, int npol_, bool inverse_only)
+        : ny(y.n), ncols(ncols_), npol(npol_), na(32 / x.r2), nb(32 / x.r1), nya(32 / y.r2), nyb(32 / y.r1) {
+        const int ways = inverse_only ? 1 : 2;
+        ca = ways * line::dft_ops(x.r1) + 5 * ways * x.r1 + 40;
+        cb = npol * (ways * line::dft_ops(x.r2) + 6 * ways * (x.r2 - 1) + 10 * ways * x.r2);
+        cya = ways * line::dft_ops(y.r1) + 15 * ways * y.r1 + 40;
+        cyb = ways * line::dft_ops(y.r2) + 6 * ways * y.r2 + 10 * ways * y.r2;
+    }
+    static int up(int a, int b) { return (a + b - 1) / b; }
+    double operator()(int nw, int L) const {
+        const int groups = up(up(ny, L), nw), cper = up(ncols, nw);
+        return groups * (up(npol * L, na) * ca + up(L, nb) * cb) + up(cper, nya) * cya + up(cper, nyb) * cyb;
+    }
+};
 
 // the shapes worth choosing from: for every (nw, L) that fits, the work of the busiest warp; a shape is dropped if
 // another has no more work and no fewer resident CTAs.  extra: further shared memory of a CTA
@@ -30,7 +37,8 @@ std::vector<PlaneShape> plane_shapes(const PWGrid& g, int prec, int npol, bool i
     const LineGeom &x = g.lines.x[prec], &y = g.lines.y[prec];
     const size_t elem = prec ? 8 : 16;
     const int maxw = line::plane_threads(elem, std::max(x.r1, y.r1)) / 32, ncols = npol * g.nxc;
-    std::vector<PlaneShape> all, out;
+    const WarpWork work(x, y, ncols, npol, inverse_only);
+    PlaneShape least[33];  // the least work of each number of resident CTAs (0: none)
     for (int nw = 1; nw <= maxw; ++nw)
         for (int L = 1; L <= 12; ++L) {
             PlaneShape s;
@@ -39,16 +47,19 @@ std::vector<PlaneShape> plane_shapes(const PWGrid& g, int prec, int npol, bool i
             s.smem = (size_t(ncols) * y.ld + size_t(nw) * npol * L * x.ld) * elem + extra;
             if (s.smem > kSmemMax) break;
             s.ctas = std::min<int>({int(228 * 1024 / (s.smem + 1024)), maxw / nw, 32});
-            s.work = warp_work(x, y, ncols, npol, nw, L, inverse_only);
-            all.push_back(s);
+            s.work = work(nw, L);
+            if (!least[s.ctas].ctas || s.work < least[s.ctas].work) least[s.ctas] = s;
         }
-    std::stable_sort(all.begin(), all.end(), [](const PlaneShape& a, const PlaneShape& b) { return a.work < b.work; });
-    int most = 0;
-    for (const PlaneShape& s : all)
-        if (s.ctas > most) {
-            most = s.ctas;
+    std::vector<PlaneShape> out;
+    for (int c = 32; c > 0; --c) {
+        const PlaneShape& s = least[c];
+        if (!s.ctas) continue;
+        // of equal work, the one with fewer warps, then fewer rows
+        if (out.empty() || s.work < out.back().work ||
+            (s.work == out.back().work && (s.nw < out.back().nw || (s.nw == out.back().nw && s.L < out.back().L))))
             out.push_back(s);
-        }
+    }
+    std::reverse(out.begin(), out.end());
     return out;
 }
 
@@ -121,17 +132,43 @@ template <typename T, typename R> OneK one_k(const PWGrid& g, int ik, int ld, co
 
 }  // namespace
 
+namespace {
+
+// The geometry of the compiled edges as constants: the search of the pads takes 5 to 20 us of a host core for a line
+// (a basis of 18^3 in 0.10 ms, with the searches of its twelve lines 0.30).
+struct EdgeGeom {
+    int n;
+    LineGeom x[2], y[2], z[2];  // y: of a square plane
+};
+template <int N> constexpr EdgeGeom edge_geom() {
+    constexpr LineGeom x0 = line::x_geom(N, 16), x1 = line::x_geom(N, 8);
+    constexpr LineGeom y0 = line::y_geom(N, 16, x0.r2), y1 = line::y_geom(N, 8, x1.r2);
+    constexpr LineGeom z0 = line::z_geom(N, 16), z1 = line::z_geom(N, 8);
+    return EdgeGeom{N, {x0, x1}, {y0, y1}, {z0, z1}};
+}
+template <int... N> struct EdgeTable { static constexpr EdgeGeom of[sizeof...(N)] = {edge_geom<N>()...}; };
+using Edges = EdgeTable<18, 20, 24, 27, 30, 32, 36, 40, 45, 48, 50, 54, 60, 64, 72, 75, 80, 81, 90, 96, 100, 108, 120, 125, 128,
+                        135, 144, 150, 160>;
+const EdgeGeom* edge_of(int n) {
+    for (const EdgeGeom& e : Edges::of)
+        if (e.n == n) return &e;
+    return nullptr;
+}
+
+}  // namespace
+
 void build_line_plan(PWGrid& g) {
     LinePlan& p = g.lines;
     p = LinePlan{};
     const int nx = g.nx, ny = g.ny, nz = g.nz;
+    const EdgeGeom *ex = edge_of(nx), *ey = edge_of(ny), *ez = edge_of(nz);
     for (int i = 0; i < 2; ++i) {
         const int elem = i ? 8 : 16;
-        p.x[i] = line::x_geom(nx, elem);
-        p.y[i] = line::y_geom(ny, elem, p.x[i].r2 ? p.x[i].r2 : 1);
-        p.z[i] = line::z_geom(nz, elem);
-        p.xbox[i] = line::z_geom(nx, elem);
-        p.ybox[i] = line::z_geom(ny, elem);
+        p.x[i] = ex ? ex->x[i] : line::x_geom(nx, elem);
+        p.y[i] = ex && nx == ny ? ex->y[i] : line::y_geom(ny, elem, p.x[i].r2 ? p.x[i].r2 : 1);
+        p.z[i] = ez ? ez->z[i] : line::z_geom(nz, elem);
+        p.xbox[i] = ex ? ex->z[i] : line::z_geom(nx, elem);
+        p.ybox[i] = ey ? ey->z[i] : line::z_geom(ny, elem);
         if (!p.x[i].r1 || !p.y[i].r1 || !p.z[i].r1) return;
     }
     // occupied x: [0, xm) and [xh, nx)

@@ -42,18 +42,16 @@ constexpr LineGeom choose_factors(int n, int elem) {
     return g;
 }
 
-// shared-memory wavefronts of one warp access by nl lanes (addresses in elements of `elem` bytes; 128 bytes a
-// wavefront, so 128 / elem lanes are served together and lanes on one bank take turns)
+// shared-memory wavefronts of one warp access by nl lanes at different addresses, in elements of `elem` bytes: 128 bytes
+// a wavefront, so 128 / elem lanes are served together and lanes on one bank take turns
 constexpr int wavefronts(const int* addr, int nl, int elem) {
     const int slots = 128 / elem;
     int total = 0;
     for (int g = 0; g < nl; g += slots) {
-        int worst = 0;
+        int on_bank[32] = {}, worst = 0;
         for (int i = g; i < nl && i < g + slots; ++i) {
-            int deg = 1;
-            for (int j = g; j < i; ++j)
-                if (addr[j] % slots == addr[i] % slots && addr[j] != addr[i]) ++deg;
-            if (deg > worst) worst = deg;
+            const int n = ++on_bank[addr[i] % slots];
+            if (n > worst) worst = n;
         }
         total += worst;
     }
@@ -63,7 +61,8 @@ constexpr int wavefronts(const int* addr, int nl, int elem) {
 constexpr double wave_cost(int r, int lp, int ip, int elem) {
     int a[32] = {};
     const int nl = 32 / r * r;
-    for (int i = 0; i < nl; ++i) a[i] = i / r * lp + i % r * ip;
+    for (int n = 0, l = 0; n < nl; ++l)
+        for (int i = 0; i < r; ++i) a[n++] = l * lp + i * ip;
     return double(wavefronts(a, nl, elem)) / nl;
 }
 // its least value (no two lanes on one bank)
@@ -82,11 +81,14 @@ constexpr LineGeom choose_pads(LineGeom g, int elem, int xr2) {
     for (int rs = g.r2; rs <= g.r2 + 3; ++rs)
         for (int ld = (g.r1 - 1) * rs + g.r2; ld <= g.r1 * rs + 8; ++ld) {
             if (best < least + 1e-3) return out;  // conflict-free, and every further candidate is larger
-            double c = 2 * wave_cost(g.r2, ld, 1, elem) + 4 * wave_cost(g.r1, ld, rs, elem) + 1e-6 * ld;
+            double c = 2 * wave_cost(g.r2, ld, 1, elem);
+            if (c < best) c += 4 * wave_cost(g.r1, ld, rs, elem);
+            c += 1e-6 * ld;
             if (xr2 && c < best) {
                 int a[32] = {};
-                const int nl = 32 / xr2 * xr2;
-                for (int i = 0; i < nl; ++i) a[i] = i / xr2 % g.r1 * rs + i / xr2 / g.r1 + i % xr2 * ld;
+                const int nl = (32 / xr2 < g.n ? 32 / xr2 : g.n) * xr2;
+                for (int n = 0, l = 0; n < nl; ++l)
+                    for (int i = 0; i < xr2; ++i) a[n++] = l % g.r1 * rs + l / g.r1 + i * ld;
                 c += 2.0 * wavefronts(a, nl, elem) / nl;
             }
             if (c < best) {
@@ -106,7 +108,9 @@ constexpr LineGeom choose_pads_z(LineGeom g, int elem) {
     for (int rs = g.r2; rs <= g.r2 + 1; ++rs)
         for (int ld = (g.r1 - 1) * rs + g.r2; ld <= g.r1 * rs + 16; ++ld) {
             if (best < least + 1e-3) return out;
-            const double c = wave_cost(g.r2, ld, 1, elem) + wave_cost(32, 0, ld, elem) + 1e-6 * ld;
+            double c = wave_cost(g.r2, ld, 1, elem);
+            if (c < best) c += wave_cost(32, 0, ld, elem);
+            c += 1e-6 * ld;
             if (c < best) {
                 best = c;
                 out.rs = rs;
