@@ -16,10 +16,13 @@ struct b200_pw_basis {
     b200::DeviceArray<float2> aux32;
     b200::DeviceArray<double2> rho_box64;  // psi(r) of one band (psi -> rho, generic grids)
     b200::DeviceArray<float2> rho_box32;
-    b200::DeviceArray<double2> rho_sb64;   // psi -> rho on the register transforms: stick buffer of a chunk,
-    b200::DeviceArray<float2> rho_sb32;    // partial rho planes, band weights
-    b200::DeviceArray<double> rho_ws64, rho_w;
-    b200::DeviceArray<float> rho_ws32;
+    // psi -> rho on the line transforms: band weights, the stick buffer of a chunk and the partial grids, one
+    // allocation sized for every smaller call too; the launch of the last chunk size of each precision
+    b200::DeviceArray<double2> rho_buf;
+    struct {
+        int chunk = 0;
+        b200::RhoShape shape;
+    } rho_plan[2];
 };
 // copy streams and events of b200_hamilt_hpsi_host, made at its first use and kept with the handle
 struct HostPipe {

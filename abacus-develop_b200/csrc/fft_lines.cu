@@ -289,17 +289,21 @@ __global__ void __launch_bounds__(256) k_rho_reduce(int nx, int ny, int nz, int 
 
 }  // namespace
 
+int rho_splits_most(const PWGrid& g, size_t elem, int nbc) {
+    const size_t grid_bytes = size_t(g.nxyz()) * (elem / 2);
+    return int(std::max<size_t>(1, std::min<size_t>(std::min(nbc, 64), kRhoPartBytes / grid_bytes)));
+}
+
 // the launch of psi -> rho for nbc bands: nsplit CTAs a plane share its bands, so that the planes of a small grid
-// fill the SMs; the partial planes take at most 512 MB
+// fill the SMs
 RhoShape rho_shape(const PWGrid& g, size_t elem, int nbc) {
-    const int prec = elem == 8;
+    const int prec = elem == 8, most = rho_splits_most(g, elem, nbc);
     const size_t real = elem / 2, plane = size_t(g.nx) * g.ny * real;
     RhoShape best;
     double bt = 1e300;
     for (const bool sums : {true, false}) {
         for (const PlaneShape& s : plane_shapes(g, prec, 1, true, sums ? plane : 0))
-            for (int ns = 1; ns <= std::min(nbc, 64); ++ns) {
-                if (ns > 1 && size_t(ns) * g.nxyz() * real > size_t(512) << 20) break;
+            for (int ns = 1; ns <= most; ++ns) {
                 // sums kept in L2 cost about a quarter more than in shared memory; a partial plane is written and read
                 const double per_band = (s.work + kStartUp / 2) * (sums ? 1.0 : 1.25);
                 const double t = double(waves(long(g.nz) * ns, s)) * (ceil_div(nbc, ns) * per_band + kStartUp) +

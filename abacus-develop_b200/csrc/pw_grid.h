@@ -183,6 +183,9 @@ struct RhoShape {
     bool sums = false;  // a CTA's sums in shared memory
 };
 RhoShape rho_shape(const PWGrid& g, size_t elem, int nbc);
+// the most partial grids rho_shape chooses for up to nbc bands (kRhoPartBytes of them where more than one)
+constexpr size_t kRhoPartBytes = size_t(128) << 20;
+int rho_splits_most(const PWGrid& g, size_t elem, int nbc);
 template <typename T, typename R>
 void launch_rho_chunk(const PWGrid& g, const RhoShape& shape, int ik, int b0, int nbc, int ld, const T* psi,
                       const double* w_chunk, T* sb, R* ws, int first, cudaStream_t s);

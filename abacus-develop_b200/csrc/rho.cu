@@ -86,9 +86,8 @@ namespace {
 using b200::guarded;
 
 template <typename T, typename R>
-void psi_to_rho(b200_pw_basis* b, b200::DeviceArray<T>& box, b200::DeviceArray<T>& aux, b200::DeviceArray<T>& sbuf,
-                b200::DeviceArray<R>& ws, int ik, int nbands, int ld, const T* psi, const double* w1, R* rho,
-                cudaStream_t s) {
+void psi_to_rho(b200_pw_basis* b, b200::DeviceArray<T>& box, b200::DeviceArray<T>& aux, int ik, int nbands, int ld,
+                const T* psi, const double* w1, R* rho, cudaStream_t s) {
     b200::PWGrid& g = b->grid;
     B200_CHECK(ik >= 0 && ik < int(g.kmaps.size()), b200::kInvalidArgument, "k-point index out of range");
     B200_CHECK(nbands >= 0 && ld >= g.kmaps[ik].npw, b200::kInvalidArgument, "ld smaller than npwk");
@@ -97,15 +96,24 @@ void psi_to_rho(b200_pw_basis* b, b200::DeviceArray<T>& box, b200::DeviceArray<T
     if (nbands > 0 && b200::lines_supported(g, sizeof(T), 1)) {
         // the same sum on the line transforms: runs of consecutive bands with a non-zero weight (the
         // reference skips the others, elecstate_pw.cpp:211), in chunks whose stick buffer is at most kStickBytes
-        b->rho_w.resize(size_t(nbands));
-        B200_CUDA(cudaMemcpyAsync(b->rho_w.ptr, w1, size_t(nbands) * sizeof(double), cudaMemcpyHostToDevice, s));
         const size_t per_band = size_t(g.nz) * g.nst;
         // (the z pass puts the bands on gridDim.y)
         const int chunk = int(std::min<size_t>(std::min(nbands, b200::kMaxGridY),
                                                std::max<size_t>(1, b200::kStickBytes / (per_band * sizeof(T)))));
-        sbuf.resize(size_t(chunk) * per_band);
-        const b200::RhoShape shape = b200::rho_shape(g, sizeof(T), chunk);
-        ws.resize(size_t(shape.nsplit) * size_t(g.nxyz()));
+        auto units = [](size_t bytes) { return (bytes + 255) / 256 * 16; };  // double2 of a part, 256-byte aligned
+        const size_t nw = units(size_t(nbands) * sizeof(double)), ns = units(size_t(chunk) * per_band * sizeof(T));
+        const size_t np = units(size_t(b200::rho_splits_most(g, sizeof(T), chunk)) * size_t(g.nxyz()) * sizeof(R));
+        b->rho_buf.resize(nw + ns + np);
+        double* w = reinterpret_cast<double*>(b->rho_buf.ptr);
+        T* sb = reinterpret_cast<T*>(b->rho_buf.ptr + nw);
+        R* ws = reinterpret_cast<R*>(b->rho_buf.ptr + nw + ns);
+        B200_CUDA(cudaMemcpyAsync(w, w1, size_t(nbands) * sizeof(double), cudaMemcpyHostToDevice, s));
+        auto& plan = b->rho_plan[sizeof(T) == 8];
+        if (plan.chunk != chunk) {
+            plan.shape = b200::rho_shape(g, sizeof(T), chunk);
+            plan.chunk = chunk;
+        }
+        const b200::RhoShape& shape = plan.shape;
         int first = 1;
         for (int b0 = 0; b0 < nbands;) {
             if (w1[b0] == 0.0) {
@@ -114,11 +122,11 @@ void psi_to_rho(b200_pw_basis* b, b200::DeviceArray<T>& box, b200::DeviceArray<T
             }
             int b1 = b0;
             while (b1 < nbands && w1[b1] != 0.0 && b1 - b0 < chunk) ++b1;
-            b200::launch_rho_chunk<T, R>(g, shape, ik, b0, b1 - b0, ld, psi, b->rho_w.ptr + b0, sbuf.ptr, ws.ptr, first, s);
+            b200::launch_rho_chunk<T, R>(g, shape, ik, b0, b1 - b0, ld, psi, w + b0, sb, ws, first, s);
             first = 0;
             b0 = b1;
         }
-        if (!first) b200::launch_rho_reduce<R>(g, shape.nsplit, ws.ptr, rho, s);
+        if (!first) b200::launch_rho_reduce<R>(g, shape.nsplit, ws, rho, s);
         return;
     }
     const long N = g.nxyz();
@@ -165,7 +173,7 @@ int b200_pw_basis_psi_to_rho_f64(b200_pw_basis* b, int ik, int nbands, int ld, c
                                  double* rho_d, void* stream) {
     return guarded([&] {
         B200_CHECK(b != nullptr, b200::kInvalidArgument, "NULL basis");
-        psi_to_rho<double2, double>(b, b->rho_box64, b->aux64, b->rho_sb64, b->rho_ws64, ik, nbands, ld,
+        psi_to_rho<double2, double>(b, b->rho_box64, b->aux64, ik, nbands, ld,
                                     (const double2*)psi_d, w1, rho_d, (cudaStream_t)stream);
     });
 }
@@ -173,7 +181,7 @@ int b200_pw_basis_psi_to_rho_f32(b200_pw_basis* b, int ik, int nbands, int ld, c
                                  float* rho_d, void* stream) {
     return guarded([&] {
         B200_CHECK(b != nullptr, b200::kInvalidArgument, "NULL basis");
-        psi_to_rho<float2, float>(b, b->rho_box32, b->aux32, b->rho_sb32, b->rho_ws32, ik, nbands, ld,
+        psi_to_rho<float2, float>(b, b->rho_box32, b->aux32, ik, nbands, ld,
                                   (const float2*)psi_d, w1, rho_d, (cudaStream_t)stream);
     });
 }

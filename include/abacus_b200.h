@@ -259,7 +259,9 @@ int b200_elecstate_pw_op_nc_f32(int domag, int domag_z, int nrxx, float w1, floa
 /* The band loop of psiToRho for k-point ik (collinear): for every band with w1[ib] != 0,
  * rho_d[r] += w1[ib] * |psi_ib(r)|^2, psi(r) = recip_to_real of band ib (psi_d + ib*ld).
  * w1: host array of nbands weights (wg(ik, ib) / omega in the reference); rho_d: nx*ny*nz in ABACUS's
- * r order, accumulated into. */
+ * r order, accumulated into.  One call at a time per basis handle, which keeps the scratch: on grids with
+ * line transforms up to 512 MB of sticks (those of nbands bands, if fewer) and 128 MB of partial densities
+ * (nbands of them, at most 64, if fewer; at least one), else two boxes of the grid. */
 int b200_pw_basis_psi_to_rho_f64(b200_pw_basis* b, int ik, int nbands, int ld, const void* psi_d, const double* w1,
                                  double* rho_d, void* stream);
 int b200_pw_basis_psi_to_rho_f32(b200_pw_basis* b, int ik, int nbands, int ld, const void* psi_d, const double* w1,

@@ -14,6 +14,30 @@ CASES = [((18, 18, 18), 1), ((20, 25, 32), 7), ((36, 36, 45), 33), ((72, 36, 50)
 
 
 @pytest.mark.gpu
+def test_band_counts_on_one_handle(pkg):
+    """The scratch of a handle serves both precisions and every band count (24 and 40 bands cut a plane into more
+    partial sums than 25 or 48): the same bits as the call on a handle of its own, in any order."""
+    torch = pytest.importorskip("torch")
+    grid = (36, 36, 36)
+    lat, k = np.diag(np.array(grid, dtype=float)), np.array([[0.125, -0.375, 0.375]])
+    rng = np.random.default_rng(6)
+
+    def basis():
+        return pkg.pwdft.PWBasisK(0.28, lat, 30.0, k, grid=grid)
+    shared = basis()
+    ld = int(shared.npwk[0])
+    psi = rng.standard_normal((48, ld)) + 1j * rng.standard_normal((48, ld))
+    w = rng.uniform(0.1, 2.0, size=48)
+
+    def rho(b, nb, prec):
+        out = torch.zeros(b.nxyz, dtype=torch.float32 if prec else torch.float64, device="cuda")
+        b.psi_to_rho(0, torch.from_numpy(psi).to("cuda", torch.complex64 if prec else torch.complex128), nb, ld, w[:nb], out)
+        return out
+    for nb, prec in ((25, 0), (24, 0), (3, 1), (40, 1), (1, 0), (48, 0), (40, 0), (48, 1), (24, 1)):
+        assert torch.equal(rho(shared, nb, prec), rho(basis(), nb, prec)), (nb, prec)
+
+
+@pytest.mark.gpu
 def test_more_bands_than_a_launch_takes(pkg):
     """A 12 x 12 x 12 grid's stick buffer holds more bands than gridDim.y: seven bands, each 10 000 times."""
     torch = pytest.importorskip("torch")
