@@ -199,6 +199,10 @@ int b200_solve_kpoints(b200_hamilt* h, int nk, const int* iks, int spin, int nba
             if (H->grid->kmaps[iks[q]].npw > H->grid->kmaps[iks[q_max]].npw) q_max = q;
         }
         const int dim_max = H->grid->kmaps[iks[q_max]].npw;
+        const int nw = std::min(nworkers, nk);
+        // the workers share the limit of a lone caller's stick buffer (whose few, well filled launches they replace by
+        // each other's), down to 48 MB each
+        const size_t stick_bytes = std::max(b200::kStickBytes / nw, size_t(48) << 20);
         std::atomic<int> next{0};
         std::mutex err_mu;
         std::exception_ptr first_err;
@@ -208,6 +212,7 @@ int b200_solve_kpoints(b200_hamilt* h, int nk, const int* iks, int spin, int nba
                 cudaStream_t s = nullptr;
                 B200_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
                 auto work = std::make_unique<b200::HpsiWork>();
+                work->stick_bytes = stick_bytes;
                 auto d = b200::make_david(nband, dim_max, david_ndim, precision, precond_d[q_max]);
                 d->set_stream(s);
                 for (int q = next.fetch_add(1); q < nk; q = next.fetch_add(1)) {
@@ -242,7 +247,6 @@ int b200_solve_kpoints(b200_hamilt* h, int nk, const int* iks, int spin, int nba
                 if (!first_err) first_err = std::current_exception();
             }
         };
-        const int nw = std::min(nworkers, nk);
         std::vector<std::thread> pool;
         for (int w = 0; w < nw; ++w) pool.emplace_back(worker);
         for (auto& t : pool) t.join();

@@ -243,7 +243,8 @@ int b200_hamilt_set_plane_variant(b200_hamilt* h, int variant);
  * Rebuilds the projector forms of every k-point (synchronous). */
 int b200_hamilt_set_fp64_gemm(b200_hamilt* h, int mode, int nmods);
 /* Bands per stick-buffer chunk of this handle's local pass (0 = the default: the largest chunk whose
- * stick buffer stays within 512 MB; 48 MB in the slots of a server).  What b200_hamilt_autotune sets.  No counterpart in the reference. */
+ * stick buffer stays within 512 MB; 512 MB shared by the workers of b200_solve_kpoints, 48 MB in the slots of
+ * a server).  What b200_hamilt_autotune sets.  No counterpart in the reference. */
 int b200_hamilt_set_band_chunk(b200_hamilt* h, int chunk);
 
 /* ---- psi -> rho (ElecStatePW::psiToRho, module_elecstate/elecstate_pw.cpp:78-216) ---- */
@@ -477,7 +478,9 @@ int b200_bpcg_stats(const b200_bpcg* d, double* max_err, int* hpsi_bands);
  * (the k loop of HSolverPW::solve, hsolver_pw.cpp:240-270, with the k-points running concurrently).
  * precision: B200_PREC_FP64 or B200_PREC_MIXED; precond_d / psi_d: host arrays of nk device pointers
  * (psi_d[q]: complex128, nband vectors at ldpsi); eigenvalues: host, nk x nband; iters: host, nk
- * (or NULL).  Each k-point's result is the same as a b200_david_diag_hamilt solve of it alone. */
+ * (or NULL).  Each k-point's result is the same as a b200_david_diag_hamilt solve of it alone.  Each worker
+ * holds a solver and an H|psi> scratch for the call; the workers' stick buffers share 512 MB in each precision
+ * used (at least 48 MB each). */
 int b200_solve_kpoints(b200_hamilt* h, int nk, const int* iks, int spin, int nband, int david_ndim, int precision,
                        const double* const* precond_d, void* const* psi_d, int ldpsi, double* eigenvalues, double thr,
                        int maxiter, int ntry_max, int notconv_max, int nworkers, int* iters);

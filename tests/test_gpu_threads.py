@@ -87,3 +87,31 @@ def test_concurrent_mixed_solves_at_96(pkg):
                                    nworkers=4)
         assert np.max(np.abs(np.asarray(eig) - np.asarray(alone))) < 1e-9
         assert list(its) == its_alone
+
+
+def test_workers_share_the_stick_buffer(pkg):
+    """64-atom sized blocks (2.6 MB of sticks a band): four workers hold 128 MB of sticks each where one takes all bands
+    in one chunk, which shows in the kernels launched; the eigenvalues are the same."""
+    P = pkg.pwdft
+    rng = np.random.default_rng(1)
+    nk, nband = 4, 96
+    b = P.PWBasisK(20.52, np.eye(3), 50.0, rng.uniform(-0.2, 0.2, size=(nk, 3)), grid=(96, 96, 96))
+    ld = int(b.npwk_max)
+    h = P.HamiltPW(b, P.PREC_FP64)
+    h.set_veff(torch.from_numpy(rng.uniform(-2.0, 0.5, size=b.nxyz)).cuda())
+    h.set_deeq([1], [1], torch.ones(1, 1, 1, 1, dtype=torch.float64, device="cuda"))
+    for ik in range(nk):
+        h.set_vkb(ik, torch.full((1, ld), 0.01 + 0j, dtype=torch.complex128, device="cuda"))
+    pcs = [P.precondition_d(b, ik) for ik in range(nk)]
+    gen = torch.Generator(device="cuda")
+    launches, eig = [], []
+    for workers in (1, 4):
+        gen.manual_seed(3)
+        x = [torch.randn(nband, ld, dtype=torch.complex128, device="cuda", generator=gen) for _ in range(nk)]
+        for ik in range(nk):
+            x[ik][:, int(b.npwk[ik]):] = 0
+        n0 = pkg._lib.load().b200_kernel_launches()
+        eig.append(h.solve_kpoints(range(nk), pcs, x, ld, nband, 1e9, 3, nworkers=workers)[0])
+        launches.append(pkg._lib.load().b200_kernel_launches() - n0)
+    assert launches[1] > launches[0]
+    assert np.max(np.abs(eig[1] - eig[0])) < 1e-9 * np.max(np.abs(eig[0]))
