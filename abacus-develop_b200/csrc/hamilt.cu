@@ -352,15 +352,15 @@ template <> struct Blas<double2> {
 };
 }  // namespace
 
-bool Hamilt::int8_products(bool ready, int nkb, int nb, int columns, int npw) const {
-    return ready && (fp64_gemm == 2 || (fp64_gemm == 1 && nb >= kOzMinBands && !proj_beats_int8(nkb, columns, npw)));
+bool Hamilt::int8_products(bool ready, int nkb, int nb, int npol, int npw) const {
+    return ready && (fp64_gemm == 2 || (fp64_gemm == 1 && nb >= kOzMinBands && !proj_beats_int8(nkb, nb, npw, npol)));
 }
 
 bool Hamilt::small_products(int ik, int nb, int nk) const {
     const NonlocalK& k = nl[ik];
     const int npw = grid->kmaps[ik].npw;
     if (fp64_gemm != 1) return false;
-    return k.oz_ready && nb >= kOzMinBands ? proj_beats_int8(k.nkb, nb, npw) : proj_small(k.nkb, nb, npw, nk);
+    return k.oz_ready && nb >= kOzMinBands ? proj_beats_int8(k.nkb, nb, npw, 1) : proj_small(k.nkb, nb, npw, nk);
 }
 
 // whether the projection of a block runs on the side stream: below about a million points of local work the two
@@ -427,7 +427,7 @@ void Hamilt::hpsi(int ik, int spin, int nb, int ld, const T* psi, T* hpsi, int m
     B200_CHECK(k.folded, kInvalidArgument, "projectors and D not both set for this k-point");
     const T* vkbd = f64 ? reinterpret_cast<const T*>(k.vkbd.ptr + size_t(spin) * nkb * k.npwx)
                         : reinterpret_cast<const T*>(k.vkbdf.ptr + size_t(spin) * nkb * k.ldf);
-    const bool oz = f64 && int8_products(k.oz_ready, nkb, nb, nb, npw);
+    const bool oz = f64 && int8_products(k.oz_ready, nkb, nb, 1, npw);
     const bool small = f64 && !oz && small_products(ik, nb, 1);
     ProjEntry pe{};
     if constexpr (f64) pe = ProjEntry{k.vkb.ptr, vkbd, psi, hpsi, npw, k.npwx};
@@ -531,15 +531,15 @@ void Hamilt::hpsi_nc(int ik, int nb, int ld, const T* psi, T* hpsi, cudaStream_t
         W.becp64.resize(size_t(2) * nkb * nb);
         becp = W.becp64.ptr;
         const bool ready = k.vkb_oz.res.ptr && k.wnc_oz[0].res.ptr;
-        const bool oz = int8_products(ready, nkb, nb, 2 * nb, npw);
+        const bool oz = int8_products(ready, nkb, nb, 2, npw);
         if (oz) {
             W.tcw.ensure();
             oz_zgemm('C', nkb, 2 * nb, npw, one, k.vkb_oz, psi, ld, zero, becp, nkb, W.ozw, W.tcw.err.ptr, s);
             for (int half = 0; half < 2; ++half)
                 oz_zgemm('N', npw, nb, 2 * nkb, one, k.wnc_oz[half], becp, 2 * nkb, one, hpsi + size_t(half) * ld, 2 * ld,
                          W.ozw, W.tcw.err.ptr, s);
-        } else if (fp64_gemm == 1 && (ready && nb >= kOzMinBands ? proj_beats_int8(nkb, 2 * nb, npw)
-                                                                 : proj_small(nkb, 2 * nb, npw, 1))) {
+        } else if (fp64_gemm == 1 && (ready && nb >= kOzMinBands ? proj_beats_int8(nkb, nb, npw, 2)
+                                                                 : proj_small_spinor(nkb, nb, npw))) {
             ProjEntry pe{k.vkb.ptr, nullptr, psi, hpsi, npw, k.npwx};
             proj_becp(&pe, 1, nkb, 2 * nb, ld, becp, W.pjw, s);
             for (int half = 0; half < 2; ++half) {

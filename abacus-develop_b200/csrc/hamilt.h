@@ -133,8 +133,8 @@ struct Hamilt {
     void hpsi_nc(int ik, int nb, int ld, const T* psi, T* hpsi, cudaStream_t s, HpsiWork* w = nullptr);
     // whether the FP64 projector products of nb bands of k-point ik (of a batch of nk) run on proj_f64.cu's kernels
     bool small_products(int ik, int nb, int nk) const;
-    // whether the products of a call of nb bands (`columns` columns of psi) run on the int8 tensor cores
-    bool int8_products(bool ready, int nkb, int nb, int columns, int npw) const;
+    // whether the products of a call of nb bands (of npol components) run on the int8 tensor cores
+    bool int8_products(bool ready, int nkb, int nb, int npol, int npw) const;
     // choose the FP64 projector products (0 cuBLAS, 1 int8 tensor cores from kOzMinBands bands, 2 int8 always;
     // nmods moduli) and re-fold
     void set_fp64_gemm(int mode, int nmods);

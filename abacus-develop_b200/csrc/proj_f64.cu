@@ -334,15 +334,37 @@ void proj_add(const ProjEntry* e, int nk, int nkb, int nb, int ld, const double2
     });
 }
 
-// One k-point: both products, B200, the library's GEMMs against these (15 us of a call are its overhead): 16 projectors
-// x 380 plane waves, 8 bands 28 / 18 us, 47 bands 35 / 19; 64 x 3000, 4 bands 30 / 21, 12 bands 26 / 27; 128 x 9240, 8
-// bands 28 / 28, 24 bands 35 / 53.  A batch saves the library's calls for every k-point: 64 x (64 x 3000), 32 bands,
-// 1.18 ms against 0.36.
-bool proj_small(int nkb, int nb, int npw, int nk) { return double(nkb) * nb * npw <= (nk > 1 ? 2e7 : 3e6); }
-// Against the int8 emulation, whose residues and recombination cost 39 ps a plane wave and band whatever the number of
-// projectors: 128 projectors x 9240, 61 bands 150 us of kernels against 81; 256 x 11 989, 64 bands 186 / 179; 256 x
-// 25 810, 64 bands 291 / 360 (these before the last waves were filled: now about a fifth less); 384 x 17 957, 48
-// bands 248 / 305.
-bool proj_beats_int8(int nkb, int nb, int npw) { return double(nkb) * nb * npw <= 2.5e8; }
+// The rules compare two estimates fitted to whole H|psi> calls of 8 to 512 projectors, 205 to 51 569 plane waves and 1
+// to 320 bands (2 623 points on B200, spinors up to 256 projectors; us, the library or the int8 emulation / these):
+//   these cost a latency that grows with the projectors (k_proj_add walks all of them; taller band tiles take longer a
+//   step) and little else in small blocks; the library's GEMMs cost a flat 10 to 20 us more than that, or, for one band, a
+//   matrix-vector product each: 16 projectors x 380 plane waves 1 band 23 / 26, 8 bands 29 / 26; 64 x 3000 2 bands 36 / 31;
+//   256 x 380 2 bands 36 / 38, 24 bands 36 / 60; 256 x 3000 2 bands 48 / 43.
+// A block of more than 3e6 products goes to the library: 128 x 9240, 8 bands 28 / 28, 24 bands 35 / 53 (products alone).
+// A batch saves the library's calls for every k-point: 64 x (64 x 3000), 32 bands 2369 / 1172; only one band of a few
+// k-points with many projectors loses: 2 x (256 x 9226) 77 / 99, 2 x (64 x 9226) 51 / 42.
+// At 6 of the points accepted the call is more than 10 % slower than with the library or the int8 emulation (with the
+// limits on the products alone at 170, up to 2.25 x), at 4 of those given up it would have been faster.
+bool proj_small(int nkb, int nb, int npw, int nk) {
+    const double products = double(nkb) * nb * npw;
+    if (nk > 1) return products <= 2e7 && (nb > 1 || nkb * (1 + 1e-4 * npw) <= 280.0 * nk - 360);
+    const int step[5] = {0, 1, 2, 4, 4};  // by band tile
+    return products <= 3e6 && nb > 1 && nkb * step[band_tiles(nb)] <= 140 + 0.05 * npw;
+}
+// Spinors: becp of 2 nb columns, then two products of 2 nkb projectors and nb bands one after the other, so the latency
+// counts twice: 16 projectors x 3000 plane waves 1 band 44 / 40, 64 x 3000 45 / 52, 256 x 380 2 bands 51 / 83.
+bool proj_small_spinor(int nkb, int nb, int npw) {
+    if (double(nkb) * 2 * nb * npw > 3e6) return false;
+    return nb == 1 ? nkb <= 16 && npw <= 30000 : nkb * (band_tiles(nb) >= 3 ? 1.5 : 1.0) <= 48 + 0.005 * npw;
+}
+// Against the int8 emulation, whose residues and recombination cost about 35 us more a call than these and a time that
+// grows with plane waves x bands whatever the number of projectors: 128 projectors x 9240, 61 bands 222 / 150; 512 x
+// 380, 64 bands 73 / 80; 512 x 3000, 128 bands 171 / 236, 48 bands 123 / 112; 256 x 9240, 96 bands 315 / 286.
+bool proj_beats_int8(int nkb, int nb, int npw, int npol) {
+    const double values = double(npw) * nb * npol, products = nkb * values;
+    if (products > 2.5e8) return false;
+    return npol == 2 ? 0.1 * nkb + 0.5e-6 * products <= 25 + 0.9e-4 * values
+                     : 0.06 * nkb + 0.28e-6 * products <= 35 + 0.5e-4 * values;
+}
 
 }  // namespace b200

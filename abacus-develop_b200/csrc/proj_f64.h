@@ -25,9 +25,10 @@ struct ProjWorkspace {
 void proj_becp(const ProjEntry* e, int nk, int nkb, int nb, int ld, double2* becp, ProjWorkspace& w, cudaStream_t s);
 // H psi += vkbd becp
 void proj_add(const ProjEntry* e, int nk, int nkb, int nb, int ld, const double2* becp, cudaStream_t s);
-// where these beat a library GEMM per product and k-point
+// where these beat a library GEMM per product and k-point: one k-point or a batch of nk; a spinor block of nb bands
 bool proj_small(int nkb, int nb, int npw, int nk);
-// where these beat the int8 emulation (gemm_oz.cu)
-bool proj_beats_int8(int nkb, int nb, int npw);
+bool proj_small_spinor(int nkb, int nb, int npw);
+// where these beat the int8 emulation (gemm_oz.cu); npol = 2: spinors
+bool proj_beats_int8(int nkb, int nb, int npw, int npol);
 
 }  // namespace b200

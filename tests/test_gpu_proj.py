@@ -53,7 +53,7 @@ def _want(b, ik, vkb, d, psi):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("nat,nh,nb", [(1, 1, 1), (1, 4, 8), (2, 8, 9), (3, 5, 16), (2, 13, 17), (5, 8, 33), (3, 18, 47),
-                                       (2, 33, 3), (2, 8, 48), (4, 9, 61), (1, 6, 130)])
+                                       (2, 33, 3), (2, 8, 48), (4, 9, 61), (1, 6, 130), (2, 18, 47), (2, 17, 31), (4, 8, 1)])
 def test_small_products(pkg, nat, nh, nb):
     torch = pytest.importorskip("torch")
     b, h, vkb, d, ld = _setup(pkg, nat, nh, 1)
