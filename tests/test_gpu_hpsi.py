@@ -33,8 +33,8 @@ def _setup(pkg, spec, kpt=None, nb=None):
 
 
 @pytest.mark.parametrize("gemm", [0, 2])  # FP64 projector products: cuBLAS ZGEMM / int8 tensor cores
-@pytest.mark.parametrize("cfg", ["si2", "diamond8", "diamond8_k", "diamond16", "diamond8_grid40", "diamond8_grid96_k",
-                                 "diamond8_grid128"])
+@pytest.mark.parametrize("cfg", ["si2", "diamond8", "diamond8_k", "diamond16", "diamond8_grid40", "diamond8_grid162",
+                                 "diamond8_grid96_k", "diamond8_grid128"])
 def test_hpsi_fp64_matches_oracle(pkg, cfg, gemm):
     S = pkg.synth
     if cfg == "si2":
@@ -45,10 +45,13 @@ def test_hpsi_fp64_matches_oracle(pkg, cfg, gemm):
         spec, kpt, nb = S.config(0), np.array([0.125, -0.375, 0.375]), 12
     elif cfg == "diamond16":
         spec, kpt, nb = S.serving_cells()[2], None, 6
-    elif cfg == "diamond8_grid40":  # a grid outside the compiled warp-transform sizes: the generic kernels
+    elif cfg == "diamond8_grid40":  # a grid of the caller's choice
         import dataclasses
         spec, kpt, nb = dataclasses.replace(S.config(0), grid=(40, 40, 40)), None, 10
-    else:  # square planes of 32*m points: the register/shuffle plane transforms
+    elif cfg == "diamond8_grid162":  # an edge that the line transforms do not cover: the Stockham kernels
+        import dataclasses
+        spec, kpt, nb = dataclasses.replace(S.config(0), grid=(36, 40, 162)), None, 10
+    else:  # larger square planes, one CTA an SM in FP64
         import dataclasses
         n = 96 if "96" in cfg else 128
         kpt = np.array([0.25, -0.125, 0.375]) if cfg.endswith("_k") else None
@@ -219,9 +222,9 @@ def test_headline_cells_match_oracle(pkg, cfg):
 @pytest.mark.parametrize("n", [64, 96, 128])
 @pytest.mark.parametrize("variant", [1, 2, 3, 4, 5])
 def test_plane_variants_match_oracle(pkg, n, variant):
-    """Every plane-pass variant of the register transforms (1: warp-shuffle lane stages; 2-5: two-pass
-    transforms through shared memory in four launch shapes) gives the oracle's local H|psi> (kinetic +
-    V_eff) on square planes of 64, 96 and 128 points, at k != 0: FP64 within 1e-12, mixed within 2e-5."""
+    """Every launch shape of the plane pass (1: the best by the library's estimate, 2-5: the next ones) gives the
+    oracle's local H|psi> (kinetic + V_eff) on square planes of 64, 96 and 128 points, at k != 0: FP64 within 1e-12,
+    mixed within 2e-5."""
     import dataclasses
     spec = dataclasses.replace(pkg.synth.config(0), grid=(n, n, n))
     wl, ref, psi, nb, ld = _setup(pkg, spec, np.array([0.25, -0.125, 0.375]), 6)

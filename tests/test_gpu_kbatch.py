@@ -67,8 +67,8 @@ def test_hpsi_kbatch_equals_per_k(pkg, mp444, prec):
 
 @pytest.mark.parametrize("prec", ["fp64", "mixed"])
 def test_hpsi_kbatch_register_transforms(pkg, prec):
-    """A 96^3 grid takes the register/shuffle transforms in both the batched and the per-k-point calls;
-    they give the same H|psi>, and one k-point agrees with the oracle."""
+    """On a 96^3 grid the batched and the per-k-point calls (line transforms, planes in shared memory one or two a SM)
+    give the same H|psi>, and one k-point agrees with the oracle."""
     spec = dataclasses.replace(pkg.synth.config(0), grid=(96, 96, 96))
     kpts = pkg.synth.mp_grid(2, True)[:3]
     P = pkg.pwdft
@@ -94,8 +94,8 @@ def test_hpsi_kbatch_register_transforms(pkg, prec):
 
 
 def test_hpsi_kbatch_generic_grid_falls_back(pkg):
-    """A grid outside the compiled warp-transform sizes takes the per-k path inside the batch call."""
-    spec = dataclasses.replace(pkg.synth.config(0), grid=(40, 40, 40))
+    """A grid with an edge that the line transforms do not cover takes the per-k path inside the batch call."""
+    spec = dataclasses.replace(pkg.synth.config(0), grid=(36, 40, 162))
     kpts = pkg.synth.mp_grid(2, True)[:3]
     P = pkg.pwdft
     wl = P.build_workload(spec, kpts=kpts)

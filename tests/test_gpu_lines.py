@@ -1,6 +1,6 @@
 """The local part of H|psi> on two-pass line transforms, every compiled edge as x, as z and on square planes,
 run-time edges, odd band counts and several k-points, against the oracle (FP64 within 1e-12 relative, FP32 within
-2e-5, the bars of test_gpu_hpsi.py), and the run descriptors it relies on on the host."""
+2e-5, the bars of test_gpu_hpsi.py).  The run descriptors it relies on: test_line_plan.py, on the host."""
 from __future__ import annotations
 
 import numpy as np

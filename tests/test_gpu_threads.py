@@ -32,22 +32,32 @@ def _run_threads(jobs):
 @pytest.mark.parametrize("prec", ["fp64", "mixed"])
 def test_local_pass_with_different_band_counts(pkg, prec):
     """Three handles of one basis, a thread and a stream each, bands 1 to 8 in different orders: bit for bit the
-    results of the same calls alone."""
+    results of the same calls alone, of the local part and of the whole H|psi> (each handle with projector scratch and
+    a second stream of its own)."""
     P = pkg.pwdft
     n = 96
     b = P.PWBasisK(0.28, np.diag([float(n)] * 3), 30.0, np.array([[0.125, -0.375, 0.375]]), grid=(n, n, n))
     rng = np.random.default_rng(4)
-    npw, ld = int(b.npwk[0]), int(b.npwk_max)
+    ld = int(b.npwk_max)
     ct = torch.complex128 if prec == "fp64" else torch.complex64
     psi = torch.from_numpy(rng.standard_normal((8, ld)) + 1j * rng.standard_normal((8, ld))).to("cuda", ct)
     veff = torch.from_numpy(rng.uniform(-2.0, 0.5, size=b.nxyz)).cuda()
     hs = [P.HamiltPW(b, P.PREC_FP64 if prec == "fp64" else P.PREC_MIXED) for _ in range(3)]
+    vkb = torch.from_numpy(rng.standard_normal((8, ld)) + 1j * rng.standard_normal((8, ld))).cuda()
+    deeq = torch.from_numpy(rng.standard_normal((1, 1, 8, 8))).cuda()
     for h in hs:
         h.set_veff(veff)
-    want = {}
-    for nb in (1, 2, 3, 4, 5, 7, 8):
-        want[nb] = torch.zeros_like(psi[:nb])
-        hs[0].hpsi_part(0, psi, want[nb], nb, ld, 1)
+        h.set_deeq([1], [8], deeq)
+        h.set_vkb(0, vkb)
+
+    def call(h, whole, nb, out):
+        if whole:
+            h.hpsi(0, psi, out, nb, ld)
+        else:
+            h.hpsi_part(0, psi, out, nb, ld, 1)
+    want = {(nb, whole): torch.zeros_like(psi[:nb]) for nb in (1, 2, 3, 4, 5, 7, 8) for whole in (False, True)}
+    for (nb, whole), out in want.items():
+        call(hs[0], whole, nb, out)
     torch.cuda.synchronize()
 
     def job(h, counts):
@@ -56,10 +66,10 @@ def test_local_pass_with_different_band_counts(pkg, prec):
             with torch.cuda.stream(s):
                 out = torch.zeros_like(psi)
                 for i in range(400):
-                    nb = counts[i % len(counts)]
-                    h.hpsi_part(0, psi, out, nb, ld, 1)
+                    nb, whole = counts[i % len(counts)], i >= 200
+                    call(h, whole, nb, out)
                     if i % 25 < len(counts):
-                        assert torch.equal(out[:nb], want[nb]), (i, nb)
+                        assert torch.equal(out[:nb], want[nb, whole]), (i, nb, whole)
                 s.synchronize()
         return run
     _run_threads([job(hs[0], (1, 5, 2)), job(hs[1], (8, 1, 4)), job(hs[2], (3, 7))])

@@ -21,6 +21,7 @@ CASES = {
     "45x45x90": (10.26, np.diag([1.0, 1.0, 2.0]), 40.0, np.zeros((1, 3)), None),
     "96^3": (20.52, np.eye(3), 50.0, np.zeros((1, 3)), None),
     "40^3_explicit": (10.26, np.eye(3), 30.0, np.zeros((1, 3)), (40, 40, 40)),
+    "36x162x40": (10.26, np.eye(3), 30.0, np.zeros((1, 3)), (36, 162, 40)),  # not on line transforms: Stockham kernels
 }
 
 

@@ -110,9 +110,9 @@ def test_gpu_psi_to_rho_sum_rule_64_atoms(pkg):
 @pytest.mark.parametrize("prec", ["f64", "f32"])
 @pytest.mark.parametrize("n", [64, 96, 128])
 def test_gpu_psi_to_rho_register_transforms_match_oracle(pkg, prec, n):
-    """The fused path (grids with register transforms: inverse z pass, then per z plane the inverse y and x
-    transforms with w|psi|^2 summed in registers, partial planes reduced in a fixed order) against the
-    oracle's band loop, at a k-point, with zero-weight bands splitting the occupied runs."""
+    """The fused path (grids with line transforms: inverse z pass, then per z plane the inverse y and x transforms with
+    w|psi|^2 summed by the same CTA, partial planes reduced in a fixed order) against the oracle's band loop, at a
+    k-point, with zero-weight bands splitting the occupied runs."""
     import dataclasses
     P = pkg.pwdft
     from oracle.pw_basis_ref import PWBasisKRef
