@@ -218,7 +218,7 @@ def ptr(t) -> int:
 
 def stream_ptr(stream=None):
     """Raw pointer of a stream, by default the current stream of the current device (read without building a
-    torch Stream object: 0.8 us instead of 3.4 on every call of a functor)."""
+    torch Stream object: 0.4 us instead of 3.4 on every call of a functor)."""
     if stream is not None:
         return stream.cuda_stream
     global _torch

@@ -304,7 +304,11 @@ RhoShape rho_shape(const PWGrid& g, size_t elem, int nbc) {
     for (const bool sums : {true, false}) {
         for (const PlaneShape& s : plane_shapes(g, prec, 1, true, sums ? plane : 0))
             for (int ns = 1; ns <= most; ++ns) {
-                // sums kept in L2 cost about a quarter more than in shared memory; a partial plane is written and read
+                // An estimate: sums kept in L2 cost a quarter more than in shared memory, and each split writes and reads
+                // a partial plane.  Measured at the best split of each (B200, shared memory / L2): 72 x 36 x 108 FP64, 96
+                // bands 246 / 312 us; 36^3 FP64, 64 bands 38.8 / 40.3; 45 x 45 x 90 81 / 84; the other way round where
+                // one CTA fills an SM: 96^3 FP64, 128 bands 766 / 675, 128^3 FP32, 160 bands 1026 / 959.  Splits: 96^3
+                // 1 1073, 3 766, 4 845, 6 769; 36^3 1 128, 4 51, 16 38.8.
                 const double per_band = (s.work + kStartUp / 2) * (sums ? 1.0 : 1.25);
                 const double t = double(waves(long(g.nz) * ns, s)) * (ceil_div(nbc, ns) * per_band + kStartUp) +
                                  0.02 * ns * double(g.nxyz()) / kSMs;

@@ -421,7 +421,7 @@ __global__ void __launch_bounds__(256) k_pad_b(int K, int N, const float2* __res
 #pragma unroll 4
     for (long n = blockIdx.y; n < N; n += gridDim.y) out[n * ldo + k] = B[n * ldb + k];
 }
-// about eight CTAs a SM, at least one column each
+// about sixteen CTAs of 256 threads a SM (two waves of those resident), at least one column each
 dim3 column_grid(int K, int N) {
     const int gx = ceil_div(K, 256);
     return dim3(gx, std::max(1, std::min(std::min(N, 65535), ceil_div(148 * 16, gx))));

@@ -100,9 +100,9 @@ struct Hamilt {
     HpsiWork work;  // default scratch for callers that do not bring their own
     int chunk_override = 0;  // bands per stick-buffer chunk chosen by the autotuner (0 = the scratch's stick_bytes)
     // FP64 projector products: 0 = cuBLAS ZGEMM; int8 tensor cores (exact modular emulation, oz_mods moduli)
-    // 1 = for calls of at least kOzMinBands bands that proj_f64.cu does not run faster (each call reads the projectors' whole residue form, twice the
-    // bytes of the FP64 projectors, so narrow calls go to cuBLAS, or if small to proj_f64.cu, whose cost scales with
-    // the bands), 2 = always
+    // 1 = for calls of at least kOzMinBands bands that proj_f64.cu does not run faster by its rule (each call reads the
+    // projectors' whole residue form, twice the bytes of the FP64 projectors, so narrow calls go to cuBLAS, or if
+    // small to proj_f64.cu, whose cost scales with the bands), 2 = always
     int fp64_gemm = 1;
     static constexpr int kOzMinBands = 48;
     int oz_mods = 16;

@@ -1,4 +1,4 @@
-// Small DFTs in registers and the radix dispatch of the two-pass line transforms (plane_g.cuh, zpass_g.cuh).
+// Small DFTs in registers and the radix dispatch of the two-pass line transforms (plane_g.cuh, box_lines.cu).
 //
 // dft<T, DIR, Q>: Q-point DFT of u[0..Q) in place, natural order in and out (DIR +1: exp(+i), -1: exp(-i)).
 // Q = 2, 3, 4, 5 direct; 6, 10, 12, 15 by the prime-factor (Good-Thomas) map, which needs no twiddles

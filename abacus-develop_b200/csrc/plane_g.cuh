@@ -1,5 +1,5 @@
 // The three passes of the local H|psi> on two-pass line transforms, for any grid whose edges factor as R1 * R2
-// (LineGeom; every 2-, 3-, 5-smooth edge from 4 to 160).
+// (LineGeom; every 2-, 3-, 5-smooth edge from 4 to 160 except 5).
 //
 // A line of n = R1 R2 points is transformed in two register passes with one exchange through shared memory:
 //   pass A  (R2 threads a line)  thread t: the R1-point DFT of f[R2 n1 + t] over n1;

@@ -124,7 +124,7 @@ template <typename T, typename R, int N, typename Src> bool z_fixed_n(const PWGr
 // the z passes with lines of nz compiled in; false for other grids (zpass_f64.cu, zpass_f32.cu, and *_many)
 template <typename T, typename R, typename Src> bool z_fixed(const PWGrid& g, const ZArgs<T, Src>& a);
 
-// the compiled edges (2-, 3-, 5-smooth, 16 to 160), split over translation units
+// the compiled edges (2-, 3-, 5-smooth, 18 to 160 except 25), split over translation units
 template <typename T, typename R>
 bool plane_fixed_a(const PWGrid& g, const PlaneShape& sh, int nplanes, const R* v, T* sb, cudaStream_t s);
 template <typename T, typename R>

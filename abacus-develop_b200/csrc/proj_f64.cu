@@ -340,7 +340,8 @@ void proj_add(const ProjEntry* e, int nk, int nkb, int nb, int ld, const double2
 //   step) and little else in small blocks; the library's GEMMs cost a flat 10 to 20 us more than that, or, for one band, a
 //   matrix-vector product each: 16 projectors x 380 plane waves 1 band 23 / 26, 8 bands 29 / 26; 64 x 3000 2 bands 36 / 31;
 //   256 x 380 2 bands 36 / 38, 24 bands 36 / 60; 256 x 3000 2 bands 48 / 43.
-// A block of more than 3e6 products goes to the library: 128 x 9240, 8 bands 28 / 28, 24 bands 35 / 53 (products alone).
+// Blocks of more than 3e6 products go to the library, which is level from there on and ahead from some 12 bands: 128 x
+// 9240, 8 bands 48 / 44, 12 bands 53 / 53, 24 bands 74 / 83; 256 x 3000, 24 bands 44 / 60.
 // A batch saves the library's calls for every k-point: 64 x (64 x 3000), 32 bands 2369 / 1172; only one band of a few
 // k-points with many projectors loses: 2 x (256 x 9226) 77 / 99, 2 x (64 x 9226) 51 / 42.
 // At 6 of the points accepted the call is more than 10 % slower than with the library or the int8 emulation (with the
@@ -358,7 +359,7 @@ bool proj_small_spinor(int nkb, int nb, int npw) {
     return nb == 1 ? nkb <= 16 && npw <= 30000 : nkb * (band_tiles(nb) >= 3 ? 1.5 : 1.0) <= 48 + 0.005 * npw;
 }
 // Against the int8 emulation, whose residues and recombination cost about 35 us more a call than these and a time that
-// grows with plane waves x bands whatever the number of projectors: 128 projectors x 9240, 61 bands 222 / 150; 512 x
+// grows with plane waves x bands whatever the number of projectors: 128 projectors x 9240, 64 bands 232 / 161; 512 x
 // 380, 64 bands 73 / 80; 512 x 3000, 128 bands 171 / 236, 48 bands 123 / 112; 256 x 9240, 96 bands 315 / 286.
 bool proj_beats_int8(int nkb, int nb, int npw, int npol) {
     const double values = double(npw) * nb * npol, products = nkb * values;

@@ -61,9 +61,9 @@ METRIC = "H|psi> bands/s (FP64) + Davidson time-to-1e-8 Ry, mixed vs FP64"
 # piece: 6 pieces of 160 bands are 16, 32, 32, 32, 32, 16)
 E2E_PIECES = (4, 5, 6, 7, 8, 10)
 # dram__bytes_read.sum + dram__bytes_write.sum of the fused local H|psi> kernels (3 launches: one band chunk
-# of all 160 bands, the autotuner's choice, x 3 passes) for one 160-band FP64 application, from an ncu
-# capture without cache flush (the local-pass traffic summary under profiles/)
-NCU_TRAFFIC_LOCAL_FP64 = 2030089984
+# of all 160 bands x 3 passes) for one 160-band FP64 application, from an ncu capture without cache flush (the
+# local-pass traffic summary under profiles/)
+NCU_TRAFFIC_LOCAL_FP64 = 2052062976
 
 
 def load_package():
@@ -607,7 +607,7 @@ def rho_bench(P, wl, psi, steps, stream):
         step()
     ms = time_steps(step, max(3, steps // 4), stream)
     return {"bands_per_s": nb / (ms * 1e-3), "ms_per_160_bands": ms,
-            "path": "register transforms: inverse z pass per band chunk, then per z plane inverse y and x transforms with w|psi|^2 summed in registers, partial planes reduced once (96^3 grid; other grids: recip_to_real per band + elecstate_pw_op, the reference's loop)"}
+            "path": "line transforms: inverse z pass per band chunk, then per z plane inverse y and x transforms with w|psi|^2 summed by the same CTA in shared memory, partial planes reduced once (grids without line transforms: recip_to_real per band + elecstate_pw_op, the reference's loop)"}
 
 
 def cpu_reference_davidson_8atom(pkg):

@@ -235,8 +235,8 @@ int b200_hamilt_set_plane_variant(b200_hamilt* h, int variant);
 /* The FP64 projector products of Nonlocal::act (nonlocal_pw.cpp:255-276, becp = vkb^H psi and
  * H psi += vkb (D becp), here with D folded into the projectors) for this handle: on the int8 tensor
  * cores (exact modular emulation of the FP64 product with nmods (12..16, default 16) moduli, as
- * b200_zgemm_i8) for H|psi> calls of at least 48 bands whose products are not small (mode 1, the default) or for every call (mode 2),
- * else cuBLAS ZGEMM (mode 0, and narrower calls in mode 1: the int8 path reads the projectors' whole
+ * b200_zgemm_i8) for H|psi> calls of at least 48 bands whose products are not small (mode 1, the default)
+ * or for every call (mode 2), else cuBLAS ZGEMM (mode 0, and narrower calls in mode 1: the int8 path reads the projectors' whole
  * residue form per call; in mode 1 small products, and batches of them, run on the library's own FP64
  * tensor-core kernels).  Modes 1 and 2 keep the projectors also in residue form (2 x nmods bytes per
  * projector entry and spin) and each H|psi> caller about 6 x nmods bytes per psi entry of scratch.
