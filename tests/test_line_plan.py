@@ -23,7 +23,7 @@ KPTS = {"gamma": [[0, 0, 0]], "k": [[0.125, -0.375, 0.375]], "edge": [[0.5, 0.5,
 
 
 @pytest.fixture(scope="module")
-def checker(tmp_path_factory):
+def plan_check(tmp_path_factory):
     spec = importlib.util.spec_from_file_location("_line_plan_build", PKG / "build.py")
     build = importlib.util.module_from_spec(spec)
     spec.loader.exec_module(build)
@@ -34,29 +34,29 @@ def checker(tmp_path_factory):
     return exe
 
 
-def _run(checker, cells):
+def _run(plan_check, cells):
     text = "".join("%s %r %s %r %d %d %d %d %s\n" % (name, lat0, " ".join(map(repr, np.asarray(lat, float).ravel().tolist())),
                                                     ecut, *grid, len(k), " ".join(map(repr, np.asarray(k, float).ravel().tolist())))
                    for name, lat0, lat, ecut, grid, k in cells)
-    r = subprocess.run([str(checker)], input=text, capture_output=True, text=True, timeout=300)
+    r = subprocess.run([str(plan_check)], input=text, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr
     return {f[0]: (int(f[1]), int(f[2])) for f in (line.split() for line in r.stdout.splitlines())}, r.stderr
 
 
-def test_runs_of_cells(checker):
+def test_runs_of_cells(plan_check):
     cells = [(f"{l}-{k}-{e}", 10.26, LATTICES[l], e, (0, 0, 0), KPTS[k]) for l in LATTICES for k in KPTS for e in (11.0, 30.0)]
-    got, err = _run(checker, cells)
+    got, err = _run(plan_check, cells)
     assert got.pop("geometry") == (1, 0), err
     assert len(got) == len(cells)
     assert all(v == (1, 0) for v in got.values()), ({n: v for n, v in got.items() if v != (1, 0)}, err)
 
 
-def test_grids_that_fall_back(checker):
+def test_grids_that_fall_back(plan_check):
     """An edge without two of the factors leaves the plan empty; a tight grid, whose runs fill whole lines, does not."""
     cells = [(f"n{n}{a}", 0.28, np.diag([float(x) for x in g]), 30.0, g, KPTS["k"])
              for n in (162, 180, 192, 216, 243) for a, g in (("x", (n, 20, 18)), ("y", (20, n, 18)), ("z", (18, 20, n)))]
     cells.append(("tight", 0.5, np.diag([24.0, 24.0, 24.0]), 30.0, (24, 24, 24), KPTS["gamma"]))
-    got, err = _run(checker, cells)
+    got, err = _run(plan_check, cells)
     got.pop("geometry")
     assert got.pop("tight") == (1, 0), err
     assert all(v == (0, 0) for v in got.values()), got
